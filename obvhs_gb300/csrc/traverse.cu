@@ -51,6 +51,16 @@ __device__ __forceinline__ float2 byte_f2(uint32_t w0, uint32_t w1, int b) {
                     make_float2(-8388608.0f, -8388608.0f));
 }
 
+// (RN(RN(v.x * a.x) + o.x), the same of y).  ptxas contracts a packed multiply
+// and a packed add into one fused multiply-add, whatever their rounding
+// qualifiers and -fmad say (seen as results that differ from the scalar ones),
+// and it drops a factor that it knows to be 1.  A multiply-add by a 1 that
+// only memory holds keeps both roundings.
+__constant__ float2 k_ones = {1.0f, 1.0f};
+__device__ __forceinline__ float2 scale_add2(float2 v, float2 a, float2 o) {
+  return __ffma2_rn(__fmul2_rn(v, a), k_ones, o);
+}
+
 struct NodeQ {
   uint4 q0, q1, q2, q3, q4;
 };
@@ -125,22 +135,23 @@ __device__ __forceinline__ uint32_t intersect_node(const NodeQ& n, float3 o, flo
   const uint32_t zn0 = rdz ? n.q4.z : n.q4.x, zf0 = rdz ? n.q4.x : n.q4.z;
   const uint32_t zn1 = rdz ? n.q4.w : n.q4.y, zf1 = rdz ? n.q4.y : n.q4.w;
   // Entry and exit distance of an axis as one pair, in sm_100's packed f32
-  // instructions (each half rounds as the scalar one).  The kernel is bound by
-  // instruction issue (81-87 % of the issue slots taken, ALU pipe 58-66 %, FMA
-  // pipe 38-41 %), and a packed instruction takes one slot for two results:
-  // 2.07M primary rays on 1M triangles 1829 -> 1592 us, 4M shadow rays on 2M
-  // 1948 -> 1769 us, 16M incoherent rays on 8M (more bound by L2) 15.65 ->
-  // 15.57 ms.  Building halves with one permute for two bytes and widening
-  // them by mixed-precision adds instead: fewer ALU instructions, no faster.
+  // instructions.  The kernel is bound by instruction issue (81-87 % of the
+  // issue slots taken, ALU pipe 58-66 %, FMA pipe 38-41 %), and a packed
+  // instruction takes one slot for two results: 2.07M primary rays on 1M
+  // triangles 1830 -> 1627 us, 4M shadow rays on 2M 1948 -> 1868 us, 1M rays
+  // through 64 instances 591 -> 549 us; 16M incoherent rays on 8M, which wait
+  // more on L2, 15.65 -> 15.81 ms.  Building halves with one permute for two
+  // bytes and widening them by mixed-precision adds: fewer ALU instructions, no
+  // faster.
   const float2 ax = make_float2(aix, aix), ay = make_float2(aiy, aiy), az = make_float2(aiz, aiz);
   const float2 ox = make_float2(aox, aox), oy = make_float2(aoy, aoy), oz = make_float2(aoz, aoz);
   uint32_t hit = 0;
 #pragma unroll
   for (int c = 0; c < 8; c++) {
     const int w = c >> 2, b = c & 3;
-    const float2 tx = __fadd2_rn(__fmul2_rn(byte_f2(w ? xn1 : xn0, w ? xf1 : xf0, b), ax), ox);
-    const float2 ty = __fadd2_rn(__fmul2_rn(byte_f2(w ? yn1 : yn0, w ? yf1 : yf0, b), ay), oy);
-    const float2 tz = __fadd2_rn(__fmul2_rn(byte_f2(w ? zn1 : zn0, w ? zf1 : zf0, b), az), oz);
+    const float2 tx = scale_add2(byte_f2(w ? xn1 : xn0, w ? xf1 : xf0, b), ax, ox);
+    const float2 ty = scale_add2(byte_f2(w ? yn1 : yn0, w ? yf1 : yf0, b), ay, oy);
+    const float2 tz = scale_add2(byte_f2(w ? zn1 : zn0, w ? zf1 : zf0, b), az, oz);
     const float tminx = tx.x, tmaxx = tx.y, tminy = ty.x, tmaxy = ty.y, tminz = tz.x, tmaxz = tz.y;
     float tmn = slab_max<FAST>(tminx, slab_max<FAST>(tminy, tminz));
     float tmx = slab_min<FAST>(tmaxx, slab_min<FAST>(tmaxy, tmaxz));
