@@ -136,6 +136,188 @@ __global__ void __launch_bounds__(BLK) k_cand_keys(const Bvh2Node* __restrict__ 
   }
 }
 
+// --- candidates of one tree sorted by one block --------------------------------
+//
+// Up to CS_MAX candidates fit one block's shared memory, so one launch computes
+// the keys, sorts them stably and writes the first `count` node ids: the key
+// launch and four digit passes over global memory cost about 5 us each at these
+// sizes, whatever they sort.  A thread keeps up to ITEMS candidates in
+// registers; warp w owns the contiguous candidates [w * 32 * I, (w + 1) * 32 *
+// I), I = ceil(n / CS_THREADS), so (warp, round, lane) is input order and the
+// passes are stable, as in k_rs_pass.
+constexpr int CS_THREADS = 1024;
+constexpr int CS_WARPS = CS_THREADS / 32;
+constexpr int CS_ITEMS = 16;
+constexpr uint32_t CS_MAX = CS_THREADS * CS_ITEMS;
+constexpr uint32_t CS_RANK_MAX = 512;  // at most this many are ranked by counting
+static_assert(CS_MAX <= 65536, "candidate indices fit 16 bits");
+
+struct CandSortSmem {
+  uint32_t wh32[CS_WARPS * 128];  // per-warp digit counts (16 bits each), then per-warp offsets
+  uint32_t part[4][256];          // per quarter of the warps: counts, then offsets
+  uint32_t base[256];             // start of each digit
+  uint32_t wsum[8];
+};
+// CandSortSmem, then the keys and the candidate indices (16 bits) of n candidates
+__host__ __device__ constexpr size_t cand_sort_smem(uint32_t n) { return sizeof(CandSortSmem) + (size_t)n * 6 + 16; }
+
+// find_candidates (src/bvh2/reinsertion.rs:121-139) for one tree by one block
+// of CS_THREADS threads: nodes first .. first + n - 1 (n <= CS_RANK_MAX) ranked
+// by counting the smaller keys, ties by index; the first `count` node ids to
+// out.  `sk`: 3 * CS_RANK_MAX words of shared memory.
+__device__ __forceinline__ void rank_candidates(const Bvh2Node* nodes, uint32_t first, uint32_t n, uint32_t count,
+                                                uint32_t* out, uint32_t* sk) {
+  const uint32_t tid = threadIdx.x;
+  uint32_t* part = sk + CS_RANK_MAX;
+  if (tid < n) sk[tid] = f32_radix_key(-half_area(node_box(ld_node(&nodes[first + tid]))));
+  __syncthreads();
+  // two threads a candidate, half of the others each
+  const uint32_t i = tid % CS_RANK_MAX, h = tid / CS_RANK_MAX, mid = (n + 1) / 2;
+  if (i < n) {
+    const uint32_t k = sk[i];
+    uint32_t below = 0;
+    for (uint32_t j = h ? mid : 0u; j < (h ? n : mid); j++) {
+      const uint32_t o = sk[j];
+      below += (o < k || (o == k && j < i)) ? 1u : 0u;
+    }
+    part[h * CS_RANK_MAX + i] = below;
+  }
+  __syncthreads();
+  if (tid < n) {
+    const uint32_t r = part[tid] + part[CS_RANK_MAX + tid];
+    if (r < count) out[r] = first + tid;
+  }
+}
+
+// The same for n <= CS_MAX: four stable 8-bit digit passes in shared memory.
+__device__ __forceinline__ void sort_candidates(const Bvh2Node* nodes, uint32_t first, uint32_t n, uint32_t count,
+                                                uint32_t* out, unsigned char* smem) {
+  CandSortSmem& sm = *reinterpret_cast<CandSortSmem*>(smem);
+  uint32_t* skey = reinterpret_cast<uint32_t*>(smem + sizeof(CandSortSmem));
+  uint16_t* sval = reinterpret_cast<uint16_t*>(skey + n);
+  uint16_t* wh_all = reinterpret_cast<uint16_t*>(sm.wh32);
+  const uint32_t tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  const uint32_t items = (n + CS_THREADS - 1) / CS_THREADS;
+  const uint32_t base_i = (uint32_t)warp * 32u * items + (uint32_t)lane;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  uint16_t* wh = wh_all + warp * 256;
+  uint32_t key[CS_ITEMS], vr[CS_ITEMS];  // vr: candidate index, rank in the warp's digit << 16
+#pragma unroll
+  for (int r = 0; r < CS_ITEMS; r++) {
+    const uint32_t i = base_i + 32u * r;
+    if ((uint32_t)r < items && i < n) {
+      key[r] = f32_radix_key(-half_area(node_box(ld_node(&nodes[first + i]))));
+      vr[r] = i;
+    }
+  }
+  for (int shift = 0; shift < 32; shift += 8) {
+#pragma unroll
+    for (int j = 0; j < CS_WARPS * 128 / CS_THREADS; j++) sm.wh32[tid + j * CS_THREADS] = 0u;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < CS_ITEMS; r++) {
+      if ((uint32_t)r >= items) break;
+      const bool valid = base_i + 32u * r < n;
+      const uint32_t d = valid ? (key[r] >> shift) & 0xffu : 256u;
+      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t lrank = __popc(peers & lt_mask);
+      const uint32_t before = valid ? wh[d] : 0u;
+      __syncwarp();
+      if (valid && lrank == 0) wh[d] = (uint16_t)(before + __popc(peers));
+      __syncwarp();
+      vr[r] = (vr[r] & 0xffffu) | (before + lrank) << 16;
+    }
+    __syncthreads();
+    {  // offsets of eight warps per thread, then of the quarters, then of the digits
+      const uint32_t d = tid & 255u, q = tid >> 8;
+      uint32_t run = 0;
+#pragma unroll
+      for (int w = 0; w < 8; w++) {
+        uint16_t* p = wh_all + (q * 8 + w) * 256 + d;
+        const uint32_t c = *p;
+        *p = (uint16_t)run;
+        run += c;
+      }
+      sm.part[q][d] = run;
+    }
+    __syncthreads();
+    uint32_t x = 0, tot = 0;
+    if (tid < 256) {
+      const uint32_t p0 = sm.part[0][tid], p1 = sm.part[1][tid], p2 = sm.part[2][tid], p3 = sm.part[3][tid];
+      sm.part[0][tid] = 0;
+      sm.part[1][tid] = p0;
+      sm.part[2][tid] = p0 + p1;
+      sm.part[3][tid] = p0 + p1 + p2;
+      tot = x = p0 + p1 + p2 + p3;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) sm.wsum[warp] = x;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t pre = 0;
+#pragma unroll
+      for (int w = 0; w < 8; w++)
+        if (w < warp) pre += sm.wsum[w];
+      sm.base[tid] = pre + x - tot;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < CS_ITEMS; r++) {
+      if ((uint32_t)r < items && base_i + 32u * r < n) {
+        const uint32_t d = (key[r] >> shift) & 0xffu;
+        const uint32_t pos = sm.base[d] + sm.part[warp >> 3][d] + wh[d] + (vr[r] >> 16);
+        skey[pos] = key[r];
+        sval[pos] = (uint16_t)vr[r];
+      }
+    }
+    __syncthreads();
+    if (shift < 24) {
+#pragma unroll
+      for (int r = 0; r < CS_ITEMS; r++) {
+        const uint32_t i = base_i + 32u * r;
+        if ((uint32_t)r < items && i < n) {
+          key[r] = skey[i];
+          vr[r] = sval[i];
+        }
+      }
+    }
+  }
+  for (uint32_t j = tid; j < count; j += CS_THREADS) out[j] = first + sval[j];
+}
+
+// One tree (cand_start null: nodes 1 .. n, the first `count` to out), or one
+// tree per block (segmented builds: scene s's nodes, its first candidates to
+// out[find_start[s]]...).
+// Dynamic shared memory of a k_cand_sort launch whose largest tree has n candidates.
+inline size_t cand_sort_bytes(uint32_t n) {
+  return n <= CS_RANK_MAX ? 3 * CS_RANK_MAX * 4 : std::max<size_t>(cand_sort_smem(n), 3 * CS_RANK_MAX * 4);
+}
+
+__global__ void __launch_bounds__(CS_THREADS, 1) k_cand_sort(const Bvh2Node* __restrict__ nodes, uint32_t n,
+                                                             uint32_t count, const uint32_t* __restrict__ cand_start,
+                                                             const uint32_t* __restrict__ find_start,
+                                                             const uint32_t* __restrict__ node_start, uint32_t* out) {
+  grid_dep_wait();
+  extern __shared__ __align__(16) unsigned char sm[];
+  uint32_t first = 1;
+  if (cand_start) {
+    const uint32_t s = blockIdx.x;
+    n = cand_start[s + 1] - cand_start[s];
+    count = find_start[s + 1] - find_start[s];
+    first = node_start[s] + 1;
+    out += find_start[s];
+  }
+  if (n <= CS_RANK_MAX)
+    rank_candidates(nodes, first, n, count, out, reinterpret_cast<uint32_t*>(sm));
+  else
+    sort_candidates(nodes, first, n, count, out, sm);
+}
+
 // find_reinsertion (src/bvh2/reinsertion.rs:233-334) for one candidate, as a
 // state machine advanced one step at a time: a stack pop of the
 // branch-and-bound search below the current pivot, or a climb to the next
@@ -327,7 +509,7 @@ struct ProposalOut {
   uint32_t* count;  // list length
 };
 
-__device__ __forceinline__ void emit_proposal(const ProposalOut& o, const uint32_t* __restrict__ parents, uint32_t k,
+__device__ __forceinline__ void emit_proposal(const ProposalOut& o, const uint32_t* parents, uint32_t k,
                                               const Reins& r) {
   o.reins[k] = r;
   if (!(r.area_diff > 0.0f)) return;
@@ -1078,6 +1260,62 @@ __global__ void __launch_bounds__(RESOLVE_THREADS) k_resolve(ResolveArgs a) {
   mark_refit_global<false>(a, P, t0, stride, gsync, st);
 }
 
+// --- whole passes of few candidates in one block -------------------------------
+//
+// A pass of at most CS_RANK_MAX candidates (half of them searched, so at most
+// eight warps of searches) leaves the GPU idle whatever its launches do; its
+// time is launches and one search's chain of dependent loads.  All such passes
+// in a row run in one launch of one block: rank the candidates, search, resolve,
+// with block barriers between them.
+constexpr uint32_t SMALL_PASSES = 32;  // per launch
+struct SmallPass {
+  uint32_t n, count, ri;  // candidates, searched, pass number
+};
+struct SmallArgs {
+  ResolveArgs ra;  // ctr: of pass 0
+  Reins* reins;
+  uint32_t cap_rt;
+  uint32_t passes;
+  SmallPass pass[SMALL_PASSES];
+};
+
+template <int CAP, bool CLAMP>
+__global__ void __launch_bounds__(RESOLVE_THREADS, 1) k_reins_small(SmallArgs a) {
+  grid_dep_wait();
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ uint32_t s_rem, s_n, s_over;
+  __shared__ uint32_t s_cand[CS_RANK_MAX];
+  static_assert(RESOLVE_THREADS == CS_THREADS, "one block does both");
+  static_assert(RESOLVE_SMEM >= 3 * CS_RANK_MAX * 4, "ranking fits the resolve's shared memory");
+  uint2 stack[CAP];
+  for (uint32_t p = 0; p < a.passes; p++) {
+    const SmallPass ps = a.pass[p];
+    ResolveArgs ra = a.ra;
+    ra.ctr = a.ra.ctr + (size_t)ps.ri * 8;
+    ra.stamp = ps.ri + 1;
+    ra.count = ps.count;
+    ra.max_rounds = ps.count + 3;
+    rank_candidates(ra.nodes, 1, ps.n, ps.count, s_cand, reinterpret_cast<uint32_t*>(sm));
+    __syncthreads();
+    if (threadIdx.x < ps.count) {
+      // (the nodes change from pass to pass: plain loads, nothing declared read-only)
+      FindSearch<CAP, CLAMP> f;
+      f.st = stack;
+      f.cap = CLAMP ? CAP : a.cap_rt;
+      f.clamp_at = 0;
+      f.start(ra.nodes, ra.parents, s_cand[threadIdx.x]);
+      while (!f.step(ra.nodes, ra.parents)) {
+      }
+      const ProposalOut po{a.reins, ra.plist, ra.conf, ra.state, ra.owner, ra.ctr};
+      emit_proposal(po, ra.parents, threadIdx.x, f.result(ra.parents, ra.status));
+    }
+    __syncthreads();
+    const uint32_t P = *(volatile uint32_t*)&ra.ctr[0];
+    if (P) resolve_block(ra, P, sm, &s_rem, &s_n, &s_over);
+    __syncthreads();
+  }
+}
+
 // Every scene's root is its own parent (k_parents covers node 0 only).
 __global__ void k_seg_root_parents(const uint32_t* __restrict__ prim_start, const uint32_t* __restrict__ node_start,
                                    uint32_t n_seg, uint32_t* __restrict__ parents) {
@@ -1151,6 +1389,31 @@ int reins_setup(BuildCtx& c, const Bvh2Node* nodes, uint32_t len, uint32_t nseq,
   return 0;
 }
 
+ResolveArgs resolve_args(BuildCtx& c, Bvh2Node* nodes, uint32_t len, uint32_t count, uint32_t ri, const ReinsBufs& B) {
+  return ResolveArgs{nodes,    B.parents, B.reins,  count, B.plist, B.conf, B.state, B.owner, B.touched, B.dirty,
+                     B.arrive, B.starts,  B.counters + 8 + (size_t)ri * 8, B.counters + 1, c.d_status, ri + 1, len,
+                     count + 3, resolve_tables_enabled() ? 1u : 0u};
+}
+
+// Passes of at most CS_RANK_MAX candidates, in order, in one launch.
+int reins_small_passes(BuildCtx& c, Bvh2Node* nodes, uint32_t len, const std::vector<SmallPass>& passes, bool clamp,
+                       uint32_t cap_rt, const ReinsBufs& B) {
+  for (size_t at = 0; at < passes.size(); at += SMALL_PASSES) {
+    SmallArgs sa;
+    sa.ra = resolve_args(c, nodes, len, 0, 0, B);
+    sa.reins = B.reins;
+    sa.cap_rt = cap_rt;
+    sa.passes = (uint32_t)std::min<size_t>(SMALL_PASSES, passes.size() - at);
+    std::copy(passes.begin() + at, passes.begin() + at + sa.passes, sa.pass);
+    if (clamp)
+      KLAUNCH("k_reins_small", launch_k(k_reins_small<192, true>, 1, RESOLVE_THREADS, RESOLVE_SMEM, c.stream, sa));
+    else
+      KLAUNCH("k_reins_small", launch_k(k_reins_small<1024, false>, 1, RESOLVE_THREADS, RESOLVE_SMEM, c.stream, sa));
+    CK(cudaGetLastError());
+  }
+  return 0;
+}
+
 // find_reinsertion for `count` candidates, then conflict resolution, moves
 // and refit (one launch each) for pass ri.  clamp: every search uses the
 // 192-entry clamped stack; else the unclamped variant with bound cap_rt, or
@@ -1189,9 +1452,7 @@ int reins_pass(BuildCtx& c, Bvh2Node* nodes, uint32_t len, const uint32_t* cand,
   }
   CK(cudaGetLastError());
   // conflict resolution, moves and refit in one launch
-  ResolveArgs ra{nodes,    B.parents, B.reins, count,  B.plist,     B.conf,     B.state,  B.owner,  B.touched,
-                 B.dirty,  B.arrive,  B.starts, pass_ctr, B.counters + 1, c.d_status, ri + 1, len, count + 3,
-                 resolve_tables_enabled() ? 1u : 0u};
+  ResolveArgs ra = resolve_args(c, nodes, len, count, ri, B);
   void* args[] = {&ra};
   uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)resolve_blocks,
                                                std::max<uint64_t>(1, div_up<uint32_t>(count, RESOLVE_THREADS)));
@@ -1208,7 +1469,13 @@ int reins_pass(BuildCtx& c, Bvh2Node* nodes, uint32_t len, const uint32_t* cand,
 }  // namespace
 
 int reinsertion_setup_kernels() {
-  return cudaFuncSetAttribute(k_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RESOLVE_SMEM) == cudaSuccess
+  return cudaFuncSetAttribute(k_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RESOLVE_SMEM) == cudaSuccess &&
+                 cudaFuncSetAttribute(k_cand_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)cand_sort_smem(CS_MAX)) == cudaSuccess &&
+                 cudaFuncSetAttribute(k_reins_small<192, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)RESOLVE_SMEM) == cudaSuccess &&
+                 cudaFuncSetAttribute(k_reins_small<1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)RESOLVE_SMEM) == cudaSuccess
              ? 0
              : -1;
 }
@@ -1261,6 +1528,7 @@ int reinsertion_device(BuildCtx& c, obvhs_bvh2* b, float batch_size_ratio, const
   const uint32_t cap_rt = b->max_depth * 2;
   if (!clamp && cap_rt > 1024) return c.fail(OBVHS_ERR_LIMIT, "reinsertion stack bound above 1024 entries");
 
+  std::vector<SmallPass> small;  // small passes not launched yet
   for (uint32_t ri = 0; ri < nseq; ri++) {
     float bsf = ((float)len * batch_size_ratio) * seq[ri];
     uint64_t batch = bsf > 0.0f ? (bsf >= 1.8446744e19f ? ~0ull : (uint64_t)bsf) : 0;
@@ -1270,7 +1538,25 @@ int reinsertion_device(BuildCtx& c, obvhs_bvh2* b, float batch_size_ratio, const
     uint32_t ncand = take - 1;
     uint32_t count = node_count - 1;
     if (count == 0) continue;
+    if (ncand <= CS_RANK_MAX) {
+      small.push_back(SmallPass{ncand, count, ri});
+      continue;
+    }
+    if (!small.empty()) {  // a custom sequence may grow again
+      r = reins_small_passes(c, b->nodes, len, small, clamp, cap_rt, B);
+      if (r) return r;
+      small.clear();
+    }
     // find_candidates
+    if (ncand <= CS_MAX) {
+      KLAUNCH("k_cand_sort", launch_k(k_cand_sort, 1, CS_THREADS, cand_sort_bytes(ncand), c.stream, b->nodes, ncand, count,
+                                      (const uint32_t*)nullptr, (const uint32_t*)nullptr, (const uint32_t*)nullptr,
+                                      vals));
+      CK(cudaGetLastError());
+      r = reins_pass(c, b->nodes, len, vals, count, ri, clamp, cap_rt, StackModes{nullptr, nullptr, 0}, B);
+      if (r) return r;
+      continue;
+    }
     uint32_t* h = chist + (size_t)(sorts & 1u) * CAND_HIST_WORDS;
     uint32_t* hn = chist + (size_t)((sorts + 1) & 1u) * CAND_HIST_WORDS;
     sorts++;
@@ -1284,6 +1570,8 @@ int reinsertion_device(BuildCtx& c, obvhs_bvh2* b, float batch_size_ratio, const
                    B);
     if (r) return r;
   }
+  r = reins_small_passes(c, b->nodes, len, small, clamp, cap_rt, B);
+  if (r) return r;
   if (applied_deferred) {
     CK(cudaMemcpyAsync(applied_deferred, B.counters + 1, 4, cudaMemcpyDeviceToHost, c.stream));
     return 0;
@@ -1312,7 +1600,7 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
   const size_t stride = 2 * ((size_t)S + 1);
   std::vector<uint32_t> tab(NSEQ * stride + S);
   uint32_t* mode = tab.data() + NSEQ * stride;
-  uint32_t tot_cand[NSEQ], tot_count[NSEQ];
+  uint32_t tot_cand[NSEQ], tot_count[NSEQ], most_cand[NSEQ] = {};
   bool all_clamp = true;
   for (uint32_t s = 0; s < S; s++) {
     const uint32_t max_depth = std::max<uint32_t>(96, h_passes[s] + 1);
@@ -1343,6 +1631,7 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
       if (node_count - 1 == 0) continue;
       ca += take - 1;
       ka += node_count - 1;
+      most_cand[ri] = std::max(most_cand[ri], take - 1);
     }
     cs[S] = ca;
     fs[S] = ka;
@@ -1373,6 +1662,14 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
     if (tot_count[ri] == 0) continue;
     const uint32_t* cs = d_tab + ri * stride;
     const uint32_t* fs = cs + S + 1;
+    if (most_cand[ri] <= CS_MAX) {  // every scene's candidates sorted by a block of their own
+      KLAUNCH("k_cand_sort", launch_k(k_cand_sort, S, CS_THREADS, cand_sort_bytes(most_cand[ri]), c.stream, nodes, 0u, 0u,
+                                      cs, fs, L.d_node_start, cand));
+      CK(cudaGetLastError());
+      r = reins_pass(c, nodes, len, cand, tot_count[ri], ri, all_clamp, 192, modes, B);
+      if (r) return r;
+      continue;
+    }
     KLAUNCH("k_seg_cand_keys", launch_k(k_seg_cand_keys, div_up<uint32_t>(tot_cand[ri], BLK), BLK, 0, c.stream,
                                    nodes, cs, L.d_node_start, S, tot_cand[ri], keys, vals));
     bool alt = false;
