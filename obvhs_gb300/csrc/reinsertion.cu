@@ -138,13 +138,18 @@ __global__ void __launch_bounds__(BLK) k_cand_keys(const Bvh2Node* __restrict__ 
 
 // --- candidates of one tree sorted by one block --------------------------------
 //
-// Up to CS_MAX candidates fit one block's shared memory, so one launch computes
-// the keys, sorts them stably and writes the first `count` node ids: the key
-// launch and four digit passes over global memory cost about 5 us each at these
-// sizes, whatever they sort.  A thread keeps up to ITEMS candidates in
-// registers; warp w owns the contiguous candidates [w * 32 * I, (w + 1) * 32 *
-// I), I = ceil(n / CS_THREADS), so (warp, round, lane) is input order and the
-// passes are stable, as in k_rs_pass.
+// Batches: up to CS_MAX candidates of a scene fit one block's shared memory, so
+// one launch computes every scene's keys, sorts them stably and writes each
+// scene's first candidates, in place of a global sort of all scenes' 64-bit
+// (scene, key) words (clear, histogram, five digit passes, gather).  Bound by
+// the block's barriers and the match / shared-memory chain of a digit pass (16
+// us for one scene of 1,000-7,000 candidates); a batch runs as many blocks as
+// scenes.  96 scenes of 1k-200k triangles 7432 -> 7010 us.  (For one tree a
+// block takes longer than the global sort above 8,000 candidates: 100k
+// triangles, slow build, 2789 -> 2894 us.)  A thread keeps up to CS_ITEMS
+// candidates in registers; warp w owns the contiguous candidates [w * 32 * I,
+// (w + 1) * 32 * I), I = ceil(n / CS_THREADS), so (warp, round, lane) is input
+// order and the passes are stable, as in k_rs_pass.
 constexpr int CS_THREADS = 1024;
 constexpr int CS_WARPS = CS_THREADS / 32;
 constexpr int CS_ITEMS = 16;
@@ -290,32 +295,23 @@ __device__ __forceinline__ void sort_candidates(const Bvh2Node* nodes, uint32_t 
   for (uint32_t j = tid; j < count; j += CS_THREADS) out[j] = first + sval[j];
 }
 
-// One tree (cand_start null: nodes 1 .. n, the first `count` to out), or one
-// tree per block (segmented builds: scene s's nodes, its first candidates to
-// out[find_start[s]]...).
 // Dynamic shared memory of a k_cand_sort launch whose largest tree has n candidates.
-inline size_t cand_sort_bytes(uint32_t n) {
-  return n <= CS_RANK_MAX ? 3 * CS_RANK_MAX * 4 : std::max<size_t>(cand_sort_smem(n), 3 * CS_RANK_MAX * 4);
-}
+inline size_t cand_sort_bytes(uint32_t n) { return std::max<size_t>(cand_sort_smem(n), 3 * CS_RANK_MAX * 4); }
 
-__global__ void __launch_bounds__(CS_THREADS, 1) k_cand_sort(const Bvh2Node* __restrict__ nodes, uint32_t n,
-                                                             uint32_t count, const uint32_t* __restrict__ cand_start,
+// One tree per block: scene s's candidates, its first ones to out[find_start[s]]...
+__global__ void __launch_bounds__(CS_THREADS, 1) k_cand_sort(const Bvh2Node* __restrict__ nodes,
+                                                             const uint32_t* __restrict__ cand_start,
                                                              const uint32_t* __restrict__ find_start,
                                                              const uint32_t* __restrict__ node_start, uint32_t* out) {
   grid_dep_wait();
   extern __shared__ __align__(16) unsigned char sm[];
-  uint32_t first = 1;
-  if (cand_start) {
-    const uint32_t s = blockIdx.x;
-    n = cand_start[s + 1] - cand_start[s];
-    count = find_start[s + 1] - find_start[s];
-    first = node_start[s] + 1;
-    out += find_start[s];
-  }
+  const uint32_t s = blockIdx.x;
+  const uint32_t n = cand_start[s + 1] - cand_start[s], k0 = find_start[s], count = find_start[s + 1] - k0;
+  const uint32_t first = node_start[s] + 1;
   if (n <= CS_RANK_MAX)
-    rank_candidates(nodes, first, n, count, out, reinterpret_cast<uint32_t*>(sm));
+    rank_candidates(nodes, first, n, count, out + k0, reinterpret_cast<uint32_t*>(sm));
   else
-    sort_candidates(nodes, first, n, count, out, sm);
+    sort_candidates(nodes, first, n, count, out + k0, sm);
 }
 
 // find_reinsertion (src/bvh2/reinsertion.rs:233-334) for one candidate, as a
@@ -589,6 +585,103 @@ __global__ void __launch_bounds__(FIND_THREADS) k_find_persistent(const Bvh2Node
       need = true;
     }
   }
+}
+
+// --- ranking and searching in one launch ----------------------------------------
+//
+// Up to RF_MAX candidates a tree: a block ranks RF_CAND of them by counting the
+// smaller keys among all (the keys of the whole tree's candidates in its shared
+// memory, eight threads a candidate, four keys a load) and searches those that
+// rank below `count`.  n^2 comparisons spread over the GPU (1-15 us) in place of
+// a key launch, four digit passes and a search launch, each of them mostly
+// launch and barrier latency at these sizes; then the longest search's chain of
+// dependent loads.  Builds: 100k triangles, medium, 1747 -> 1413 us; 30k 1256
+// -> 942; 300k 2572 -> 2280; 100k, slow, 2789 -> 2528; 20 scenes of 2k-50k 2977
+// -> 2451 us.
+// The line at RF_MAX: with 8,192 instead the 300k build takes 2344 us, with
+// 4,096 2419; above 16,384 the keys leave room for two blocks an SM and the
+// comparisons grow past the sort's time.  RF_PAIRS, the comparisons of a batch's
+// launch: 64M keeps 96 scenes at 7028 us; 256M 7086, 1,024M 7206.
+constexpr int RF_THREADS = 512;
+constexpr uint32_t RF_CAND = 64;
+constexpr uint32_t RF_SLICES = RF_THREADS / RF_CAND;
+constexpr uint32_t RF_MAX = 16384;
+constexpr uint64_t RF_PAIRS = 64ull << 20;  // comparisons of a launch over many trees
+
+// Several trees in one launch: their tables (block b ranks chunk b -
+// chunk_start[s] of scene s); all null for one tree.
+struct RankSegs {
+  const uint32_t* chunk_start;
+  const uint32_t* cand_start;
+  const uint32_t* find_start;
+  const uint32_t* node_start;
+  uint32_t n_seg;
+};
+
+template <int CAP, bool CLAMP>
+__global__ void __launch_bounds__(RF_THREADS) k_rank_find(const Bvh2Node* __restrict__ nodes,
+                                                          const uint32_t* __restrict__ parents, uint32_t n,
+                                                          uint32_t count, uint32_t cap_rt, ProposalOut out,
+                                                          uint32_t* status, StackModes modes, RankSegs segs) {
+  grid_dep_wait();
+  extern __shared__ __align__(16) uint32_t s_key[];
+  __shared__ uint32_t s_part[RF_SLICES][RF_CAND];
+  __shared__ uint2 s_list[RF_CAND];
+  __shared__ uint32_t s_found;
+  const uint32_t tid = threadIdx.x;
+  uint32_t first = 1, i0 = blockIdx.x * RF_CAND, k0 = 0;
+  if (segs.chunk_start) {
+    const uint32_t s = seg_find(segs.chunk_start, segs.n_seg, blockIdx.x);
+    i0 = (blockIdx.x - __ldg(&segs.chunk_start[s])) * RF_CAND;
+    n = __ldg(&segs.cand_start[s + 1]) - __ldg(&segs.cand_start[s]);
+    k0 = __ldg(&segs.find_start[s]);
+    count = __ldg(&segs.find_start[s + 1]) - k0;
+    first = __ldg(&segs.node_start[s]) + 1;
+  }
+  for (uint32_t j = tid; j < n; j += RF_THREADS) s_key[j] = f32_radix_key(-half_area(node_box(ld_node(&nodes[first + j]))));
+  if (tid == 0) s_found = 0;
+  __syncthreads();
+  // candidate i0 + c against slice h of the keys: before the block's own
+  // candidates an equal key is smaller, after them it is not
+  const uint32_t c = tid % RF_CAND, h = tid / RF_CAND, i = i0 + c;
+  if (i < n) {
+    const uint32_t per = ((n + RF_SLICES - 1) / RF_SLICES + 3) & ~3u;
+    const uint32_t lo = min(h * per, n), hi = min(lo + per, n);
+    const uint32_t own_lo = min(max(i0, lo), hi), own_hi = min(max(i0 + RF_CAND, lo), hi);
+    const uint32_t k = s_key[i];
+    uint32_t below = 0, j = lo;
+    for (; j + 4 <= own_lo; j += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(&s_key[j]);
+      below += (q.x <= k) + (q.y <= k) + (q.z <= k) + (q.w <= k);
+    }
+    for (; j < own_lo; j++) below += s_key[j] <= k;
+    for (; j < own_hi; j++) below += s_key[j] < k || (s_key[j] == k && j < i);
+    for (; j < hi && (j & 3u); j++) below += s_key[j] < k;
+    for (; j + 4 <= hi; j += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(&s_key[j]);
+      below += (q.x < k) + (q.y < k) + (q.z < k) + (q.w < k);
+    }
+    for (; j < hi; j++) below += s_key[j] < k;
+    s_part[h][c] = below;
+  }
+  __syncthreads();
+  if (tid < RF_CAND && i < n) {
+    uint32_t r = 0;
+#pragma unroll
+    for (int q = 0; q < (int)RF_SLICES; q++) r += s_part[q][tid];
+    if (r < count) s_list[atomicAdd(&s_found, 1u)] = make_uint2(first + i, k0 + r);
+  }
+  __syncthreads();
+  if (tid >= s_found) return;
+  const uint2 mine = s_list[tid];
+  uint2 stack[CAP];
+  FindSearch<CAP, CLAMP> f;
+  f.st = stack;
+  set_stack_mode(f, cap_rt, modes, mine.x);
+  f.start(nodes, parents, mine.x);
+  while (!f.step(nodes, parents)) {
+  }
+  emit_proposal(out, parents, mine.y, f.result(parents, status));
 }
 
 struct ResolveArgs {
@@ -1266,7 +1359,9 @@ __global__ void __launch_bounds__(RESOLVE_THREADS) k_resolve(ResolveArgs a) {
 // eight warps of searches) leaves the GPU idle whatever its launches do; its
 // time is launches and one search's chain of dependent loads.  All such passes
 // in a row run in one launch of one block: rank the candidates, search, resolve,
-// with block barriers between them.
+// with block barriers between them (2k triangles, fast: 16 passes in 44 us; the
+// build 782 -> 501 us).  The line lies where the searches would fill more than
+// two warps of each of the SM's schedulers.
 constexpr uint32_t SMALL_PASSES = 32;  // per launch
 struct SmallPass {
   uint32_t n, count, ri;  // candidates, searched, pass number
@@ -1395,6 +1490,47 @@ ResolveArgs resolve_args(BuildCtx& c, Bvh2Node* nodes, uint32_t len, uint32_t co
                      count + 3, resolve_tables_enabled() ? 1u : 0u};
 }
 
+// Conflict resolution, moves and refit for pass ri, whose searches (`count`
+// of them) have listed their proposals.
+int reins_resolve(BuildCtx& c, Bvh2Node* nodes, uint32_t len, uint32_t count, uint32_t ri, const ReinsBufs& B) {
+  static std::atomic<int> resolve_per_sm_s{0};
+  int resolve_per_sm = resolve_per_sm_s.load();
+  if (!resolve_per_sm) {
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resolve_per_sm, k_resolve, RESOLVE_THREADS, RESOLVE_SMEM));
+    resolve_per_sm = std::max(1, resolve_per_sm);
+    resolve_per_sm_s.store(resolve_per_sm);
+  }
+  const int resolve_blocks = resolve_per_sm * c.num_sms;
+  ResolveArgs ra = resolve_args(c, nodes, len, count, ri, B);
+  void* args[] = {&ra};
+  uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)resolve_blocks,
+                                               std::max<uint64_t>(1, div_up<uint32_t>(count, RESOLVE_THREADS)));
+  if (grid == 1 || count <= RESOLVE_SINGLE_MAX || gpu_shared(c)) {
+    // one block, a normal launch (block barriers only)
+    KLAUNCH("k_resolve", launch_k(k_resolve, 1, RESOLVE_THREADS, RESOLVE_SMEM, c.stream, ra));
+  } else {
+    KLAUNCH("k_resolve", CK(coop_launch(c, (const void*)k_resolve, grid, RESOLVE_THREADS, args, RESOLVE_SMEM)));
+  }
+  CK(cudaGetLastError());
+  return 0;
+}
+
+// A pass of trees with at most RF_MAX candidates each (the largest has
+// max_n): `blocks` blocks rank and search, then the resolution.
+int reins_rank_pass(BuildCtx& c, Bvh2Node* nodes, uint32_t len, uint32_t n, uint32_t count, uint32_t max_n,
+                    uint32_t blocks, uint32_t ri, bool clamp, uint32_t cap_rt, StackModes modes, RankSegs segs,
+                    const ReinsBufs& B) {
+  const ProposalOut po{B.reins, B.plist, B.conf, B.state, B.owner, B.counters + 8 + (size_t)ri * 8};
+  if (clamp)
+    KLAUNCH("k_rank_find", launch_k(k_rank_find<192, true>, blocks, RF_THREADS, (size_t)max_n * 4 + 16, c.stream, nodes,
+                                    B.parents, n, count, cap_rt, po, c.d_status, modes, segs));
+  else
+    KLAUNCH("k_rank_find", launch_k(k_rank_find<1024, false>, blocks, RF_THREADS, (size_t)max_n * 4 + 16, c.stream, nodes,
+                                    B.parents, n, count, cap_rt, po, c.d_status, modes, segs));
+  CK(cudaGetLastError());
+  return reins_resolve(c, nodes, len, count, ri, B);
+}
+
 // Passes of at most CS_RANK_MAX candidates, in order, in one launch.
 int reins_small_passes(BuildCtx& c, Bvh2Node* nodes, uint32_t len, const std::vector<SmallPass>& passes, bool clamp,
                        uint32_t cap_rt, const ReinsBufs& B) {
@@ -1420,19 +1556,14 @@ int reins_small_passes(BuildCtx& c, Bvh2Node* nodes, uint32_t len, const std::ve
 // per-tree modes when `modes.mode` is set.
 int reins_pass(BuildCtx& c, Bvh2Node* nodes, uint32_t len, const uint32_t* cand, uint32_t count, uint32_t ri,
                bool clamp, uint32_t cap_rt, StackModes modes, const ReinsBufs& B) {
-  static std::atomic<int> find_per_sm_s{0}, resolve_per_sm_s{0};
-  int find_per_sm = find_per_sm_s.load(), resolve_per_sm = resolve_per_sm_s.load();
+  static std::atomic<int> find_per_sm_s{0};
+  int find_per_sm = find_per_sm_s.load();
   if (!find_per_sm) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&find_per_sm, k_find_persistent<192, true>, FIND_THREADS, 0));
     find_per_sm = std::max(1, find_per_sm);
     find_per_sm_s.store(find_per_sm);
   }
-  if (!resolve_per_sm) {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resolve_per_sm, k_resolve, RESOLVE_THREADS, RESOLVE_SMEM));
-    resolve_per_sm = std::max(1, resolve_per_sm);
-    resolve_per_sm_s.store(resolve_per_sm);
-  }
-  const int find_blocks = find_per_sm * c.num_sms, resolve_blocks = resolve_per_sm * c.num_sms;
+  const int find_blocks = find_per_sm * c.num_sms;
   uint32_t* pass_ctr = B.counters + 8 + (size_t)ri * 8;  // [5]: next candidate for k_find
   const uint32_t fblocks = div_up<uint32_t>(count, FIND_THREADS);
   const ProposalOut po{B.reins, B.plist, B.conf, B.state, B.owner, pass_ctr};
@@ -1451,19 +1582,7 @@ int reins_pass(BuildCtx& c, Bvh2Node* nodes, uint32_t len, const uint32_t* cand,
                                                                              po, c.d_status, modes));
   }
   CK(cudaGetLastError());
-  // conflict resolution, moves and refit in one launch
-  ResolveArgs ra = resolve_args(c, nodes, len, count, ri, B);
-  void* args[] = {&ra};
-  uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)resolve_blocks,
-                                               std::max<uint64_t>(1, div_up<uint32_t>(count, RESOLVE_THREADS)));
-  if (grid == 1 || count <= RESOLVE_SINGLE_MAX || gpu_shared(c)) {
-    // one block, a normal launch (block barriers only)
-    KLAUNCH("k_resolve", launch_k(k_resolve, 1, RESOLVE_THREADS, RESOLVE_SMEM, c.stream, ra));
-  } else {
-    KLAUNCH("k_resolve", CK(coop_launch(c, (const void*)k_resolve, grid, RESOLVE_THREADS, args, RESOLVE_SMEM)));
-  }
-  CK(cudaGetLastError());
-  return 0;
+  return reins_resolve(c, nodes, len, count, ri, B);
 }
 
 }  // namespace
@@ -1472,6 +1591,10 @@ int reinsertion_setup_kernels() {
   return cudaFuncSetAttribute(k_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RESOLVE_SMEM) == cudaSuccess &&
                  cudaFuncSetAttribute(k_cand_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)cand_sort_smem(CS_MAX)) == cudaSuccess &&
+                 cudaFuncSetAttribute(k_rank_find<192, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)RF_MAX * 4 + 16) == cudaSuccess &&
+                 cudaFuncSetAttribute(k_rank_find<1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)RF_MAX * 4 + 16) == cudaSuccess &&
                  cudaFuncSetAttribute(k_reins_small<192, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)RESOLVE_SMEM) == cudaSuccess &&
                  cudaFuncSetAttribute(k_reins_small<1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1548,12 +1671,9 @@ int reinsertion_device(BuildCtx& c, obvhs_bvh2* b, float batch_size_ratio, const
       small.clear();
     }
     // find_candidates
-    if (ncand <= CS_MAX) {
-      KLAUNCH("k_cand_sort", launch_k(k_cand_sort, 1, CS_THREADS, cand_sort_bytes(ncand), c.stream, b->nodes, ncand, count,
-                                      (const uint32_t*)nullptr, (const uint32_t*)nullptr, (const uint32_t*)nullptr,
-                                      vals));
-      CK(cudaGetLastError());
-      r = reins_pass(c, b->nodes, len, vals, count, ri, clamp, cap_rt, StackModes{nullptr, nullptr, 0}, B);
+    if (ncand <= RF_MAX) {
+      r = reins_rank_pass(c, b->nodes, len, ncand, count, ncand, div_up<uint32_t>(ncand, RF_CAND), ri, clamp, cap_rt,
+                          StackModes{nullptr, nullptr, 0}, RankSegs{nullptr, nullptr, nullptr, nullptr, 0}, B);
       if (r) return r;
       continue;
     }
@@ -1596,11 +1716,12 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
   const uint32_t S = L.n_seg, len = L.n_slots;
   if (len == 0 || !(ratio > 0.0f)) return 0;
   constexpr uint32_t NSEQ = 16;
-  // per pass: cand_start[S + 1], find_start[S + 1]; per scene: stack mode
-  const size_t stride = 2 * ((size_t)S + 1);
+  // per pass: cand_start[S + 1], find_start[S + 1], chunk_start[S + 1]; per scene: stack mode
+  const size_t stride = 3 * ((size_t)S + 1);
   std::vector<uint32_t> tab(NSEQ * stride + S);
   uint32_t* mode = tab.data() + NSEQ * stride;
   uint32_t tot_cand[NSEQ], tot_count[NSEQ], most_cand[NSEQ] = {};
+  uint64_t pairs[NSEQ] = {};  // comparisons that ranking would take
   bool all_clamp = true;
   for (uint32_t s = 0; s < S; s++) {
     const uint32_t max_depth = std::max<uint32_t>(96, h_passes[s] + 1);
@@ -1615,11 +1736,13 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
   for (uint32_t ri = 0; ri < NSEQ; ri++) {
     uint32_t* cs = tab.data() + ri * stride;
     uint32_t* fs = cs + S + 1;
+    uint32_t* ch = fs + S + 1;
     const float q = 1.0f / (float)(2 * ri + 1);
-    uint32_t ca = 0, ka = 0;
+    uint32_t ca = 0, ka = 0, cha = 0;
     for (uint32_t s = 0; s < S; s++) {
       cs[s] = ca;
       fs[s] = ka;
+      ch[s] = cha;
       const uint32_t m = L.leaves(s);
       if (m < 2) continue;
       const uint32_t n = 2 * m - 1;
@@ -1631,10 +1754,13 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
       if (node_count - 1 == 0) continue;
       ca += take - 1;
       ka += node_count - 1;
+      cha += div_up<uint32_t>(take - 1, RF_CAND);
       most_cand[ri] = std::max(most_cand[ri], take - 1);
+      pairs[ri] += (uint64_t)(take - 1) * (take - 1);
     }
     cs[S] = ca;
     fs[S] = ka;
+    ch[S] = cha;
     tot_cand[ri] = ca;
     tot_count[ri] = ka;
   }
@@ -1662,9 +1788,16 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
     if (tot_count[ri] == 0) continue;
     const uint32_t* cs = d_tab + ri * stride;
     const uint32_t* fs = cs + S + 1;
+    if (most_cand[ri] <= RF_MAX && pairs[ri] <= RF_PAIRS) {
+      const uint32_t* ch = fs + S + 1;
+      r = reins_rank_pass(c, nodes, len, 0, tot_count[ri], most_cand[ri], tab[ri * stride + 2 * ((size_t)S + 1) + S], ri,
+                          all_clamp, 192, modes, RankSegs{ch, cs, fs, L.d_node_start, S}, B);
+      if (r) return r;
+      continue;
+    }
     if (most_cand[ri] <= CS_MAX) {  // every scene's candidates sorted by a block of their own
-      KLAUNCH("k_cand_sort", launch_k(k_cand_sort, S, CS_THREADS, cand_sort_bytes(most_cand[ri]), c.stream, nodes, 0u, 0u,
-                                      cs, fs, L.d_node_start, cand));
+      KLAUNCH("k_cand_sort", launch_k(k_cand_sort, S, CS_THREADS, cand_sort_bytes(most_cand[ri]), c.stream, nodes, cs, fs,
+                                      L.d_node_start, cand));
       CK(cudaGetLastError());
       r = reins_pass(c, nodes, len, cand, tot_count[ri], ri, all_clamp, 192, modes, B);
       if (r) return r;

@@ -1,6 +1,7 @@
 """Reinsertion passes whose candidates one block ranks (512 and fewer, whole
-passes in one launch) or sorts (16,384 and fewer), and the global sort above,
-at the sizes where one gives way to the next: the oracle's tree bit for bit.
+passes in one launch) or many blocks (16,384 and fewer), and the global sort
+above, at the sizes where one gives way to the next: the oracle's tree bit for
+bit.  Batches: one block per scene sorts above 64M comparisons a launch.
 Copies of one box give equal areas and gains, whose order is the candidates'
 input order."""
 import numpy as np
@@ -68,8 +69,8 @@ def test_unclamped_stack(G):
 
 @pytest.mark.parametrize("sizes", [[2, 3, 700, 150_000, 30], [300, 90_000, 5_000, 1]])
 def test_segmented_candidate_sorts(G, sizes):
-    """Scenes whose candidates one block sorts beside scenes whose first
-    passes are above that, each equal to the scene built alone."""
+    """Scenes whose first passes take the global sort, then a block per scene,
+    then the ranking, each equal to the scene built alone."""
     p = BvhBuildParams.medium_build()
     tris = [S.scene2_tris(n, offset=i) for i, n in enumerate(sizes)]
     for cw, t in zip(G.build_cwbvh_from_tris_segmented(tris, p), tris):
