@@ -1103,9 +1103,11 @@ __global__ void __launch_bounds__(COOP_GROUPS * PT, 1) k_ploc_coop(PlocCoopArgs 
 // tile table (scene s has ceil(count_s / chunk) tiles when count_s > 1) from
 // the per-scene counts, and the tiles of all scenes are spread over the
 // groups as in k_ploc_coop; a tile's output offsets count only the earlier
-// tiles of its own scene.  A scene whose count reaches 1 writes its root to
-// out[node_start[s]] and drops out.  No tail kernel: the loop runs until
-// every scene is done.
+// tiles of its own scene.  A scene drops out once at most SEG_TAIL_MAX of its
+// clusters are live (its clusters stay in the buffer of its pass parity), and
+// k_ploc_seg_tail finishes it.
+constexpr uint32_t SEG_TAIL_MAX = TAIL_MAX;
+constexpr int SEG_TAIL_THREADS = 1024;
 constexpr uint32_t SEG_MAX = OBVHS_SEG_MAX_SCENES;  // scenes per launch (tile table in shared memory)
 
 struct PlocSegArgs {
@@ -1214,10 +1216,17 @@ __global__ void __launch_bounds__(COOP_GROUPS * PT, 1) k_ploc_seg(PlocSegArgs a)
         tstart, S,
         [&](uint32_t s) {
           const uint32_t c = __ldcg(&cnt[s]);
-          return c > 1 ? div_up<uint32_t>(c, chunk) : 0u;
+          return c > SEG_TAIL_MAX ? div_up<uint32_t>(c, chunk) : 0u;
         },
         s_warp);
     const uint32_t ntiles = tstart[S];
+    // a scene left to the tail has the same count in both parities, so it gets
+    // no tiles again (nothing else reads or writes the other parity's word now)
+    if (blockIdx.x == 0)
+      for (uint32_t s = threadIdx.x; s < S; s += COOP_GROUPS * PT) {
+        const uint32_t c = __ldcg(&cnt[s]);
+        if (c <= SEG_TAIL_MAX) a.count[(size_t)(parity ^ 1) * S + s] = c;
+      }
 
     // A: merge offsets and tile counts
     for (uint32_t tile = first_tile; tile < ntiles; tile += tile_step) {
@@ -1241,16 +1250,8 @@ __global__ void __launch_bounds__(COOP_GROUPS * PT, 1) k_ploc_seg(PlocSegArgs a)
           a.count[(size_t)(parity ^ 1) * S + s] = tot.x;
           a.insert[(size_t)(parity ^ 1) * S + s] = ins_top - 2 * tot.y;
           atomicAdd(&a.sum_counts[s], (unsigned long long)count);
-          if (tot.x > 1) {
-            atomicAdd(&a.ctl[1 + (parity ^ 1)], tot.x);
-          } else {
-            a.count[(size_t)parity * S + s] = tot.x;  // done: 1 in both parities
-            a.passes[s] = pass + 1;
-          }
-        }
-        if (tot.x == 1) {  // one tile (a pass at most halves the count): the root is next[0]
-          group_sync(group);
-          if (tid == 0) st_node(&a.out[__ldg(&a.node_start[s])], ld_node_cg(&next[cb]));
+          a.passes[s] = pass + 1;
+          if (tot.x > SEG_TAIL_MAX) atomicAdd(&a.ctl[1 + (parity ^ 1)], tot.x);
         }
       }
     }
@@ -1277,7 +1278,7 @@ __global__ void k_ploc_seg_init(const Bvh2Node* __restrict__ cur, const uint32_t
   sum_counts[s] = 0;
   if (m >= 1) st_node(&out[nb + 2 * m - 1], make_node(Box{}, 0, SEG_PAD_CHILD));
   if (m == 1) st_node(&out[nb], ld_node(&cur[prim_start[s]]));
-  if (m > 1) atomicAdd(&ctl[1], m);
+  if (m > SEG_TAIL_MAX) atomicAdd(&ctl[1], m);
 }
 
 // --- single-CTA tail ---------------------------------------------------------
@@ -1285,39 +1286,42 @@ __global__ void k_ploc_seg_init(const Bvh2Node* __restrict__ cur, const uint32_t
 constexpr int TAIL_THREADS = 1024;
 
 // The tail keeps its clusters as structures of arrays: eight word arrays of
-// TAIL_MAX (min x, y, z, prim count, max x, y, z, first index), so lanes that
+// CAP (min x, y, z, prim count, max x, y, z, first index), so lanes that
 // read consecutive clusters read consecutive words (no bank conflicts).
+template <uint32_t CAP>
 __device__ __forceinline__ Box sbox(const float* s, uint32_t j) {
-  return Box{make_float3(s[j], s[TAIL_MAX + j], s[2 * TAIL_MAX + j]),
-             make_float3(s[4 * TAIL_MAX + j], s[5 * TAIL_MAX + j], s[6 * TAIL_MAX + j])};
+  return Box{make_float3(s[j], s[CAP + j], s[2 * CAP + j]),
+             make_float3(s[4 * CAP + j], s[5 * CAP + j], s[6 * CAP + j])};
 }
+template <uint32_t CAP>
 __device__ __forceinline__ void snode_get(const float* s, uint32_t j, float4& a, float4& b) {
-  a = make_float4(s[j], s[TAIL_MAX + j], s[2 * TAIL_MAX + j], s[3 * TAIL_MAX + j]);
-  b = make_float4(s[4 * TAIL_MAX + j], s[5 * TAIL_MAX + j], s[6 * TAIL_MAX + j], s[7 * TAIL_MAX + j]);
+  a = make_float4(s[j], s[CAP + j], s[2 * CAP + j], s[3 * CAP + j]);
+  b = make_float4(s[4 * CAP + j], s[5 * CAP + j], s[6 * CAP + j], s[7 * CAP + j]);
 }
+template <uint32_t CAP>
 __device__ __forceinline__ void snode_put(float* s, uint32_t j, const float4& a, const float4& b) {
   s[j] = a.x;
-  s[TAIL_MAX + j] = a.y;
-  s[2 * TAIL_MAX + j] = a.z;
-  s[3 * TAIL_MAX + j] = a.w;
-  s[4 * TAIL_MAX + j] = b.x;
-  s[5 * TAIL_MAX + j] = b.y;
-  s[6 * TAIL_MAX + j] = b.z;
-  s[7 * TAIL_MAX + j] = b.w;
+  s[CAP + j] = a.y;
+  s[2 * CAP + j] = a.z;
+  s[3 * CAP + j] = a.w;
+  s[4 * CAP + j] = b.x;
+  s[5 * CAP + j] = b.y;
+  s[6 * CAP + j] = b.z;
+  s[7 * CAP + j] = b.w;
 }
 
 // The tail's neighbour search: sm[i] = offset of cluster i's best neighbour.
-template <bool FAST>
+template <uint32_t CAP, int THREADS, bool FAST>
 __device__ __forceinline__ void tail_search(const float* cur, uint32_t count, bool d1, int r, int8_t* sm, int tid) {
-  for (uint32_t i = tid; i < count; i += TAIL_THREADS) {
-    Box me = sbox(cur, i);
+  for (uint32_t i = tid; i < count; i += THREADS) {
+    Box me = sbox<CAP>(cur, i);
     int8_t m;
     if (d1) {
       if (i == count - 1) {
         m = -1;
       } else {
-        float c = pair_cost<FAST>(me, sbox(cur, i + 1));
-        float last = i == 0 ? __int_as_float(0x7f800000) : pair_cost<FAST>(sbox(cur, i - 1), me);
+        float c = pair_cost<FAST>(me, sbox<CAP>(cur, i + 1));
+        float last = i == 0 ? __int_as_float(0x7f800000) : pair_cost<FAST>(sbox<CAP>(cur, i - 1), me);
         m = last < c ? -1 : 1;
       }
     } else {
@@ -1326,14 +1330,14 @@ __device__ __forceinline__ void tail_search(const float* cur, uint32_t count, bo
       uint32_t best = i;
       float bc = __int_as_float(0x7f800000);
       for (uint32_t j = begin; j < i; j++) {
-        float c = pair_cost<FAST>(sbox(cur, j), me);
+        float c = pair_cost<FAST>(sbox<CAP>(cur, j), me);
         if (c <= bc) {
           best = j;
           bc = c;
         }
       }
       for (uint32_t j = i + 1; j < end; j++) {
-        float c = pair_cost<FAST>(me, sbox(cur, j));
+        float c = pair_cost<FAST>(me, sbox<CAP>(cur, j));
         if (c <= bc) {
           best = j;
           bc = c;
@@ -1345,44 +1349,35 @@ __device__ __forceinline__ void tail_search(const float* cur, uint32_t count, bo
   }
 }
 
-// Finishes every remaining pass (count <= TAIL_MAX) inside one CTA.
-// The live clusters are in buf[passes & 1].
-__global__ void __launch_bounds__(TAIL_THREADS) k_ploc_tail(const Bvh2Node* __restrict__ buf0,
-                                                            const Bvh2Node* __restrict__ buf1, PlocState* st,
-                                                            int radius, uint32_t depth_threshold, uint32_t max_passes,
-                                                            Bvh2Node* __restrict__ out, uint32_t* status,
-                                                            const uint32_t* __restrict__ remap, int fast,
-                                                            uint32_t* pass_ins) {
-  grid_dep_wait();
-  extern __shared__ float4 smem[];
-  float* sa = reinterpret_cast<float*>(smem);  // TAIL_MAX clusters (8 word arrays)
-  float* sb = sa + 8 * TAIL_MAX;               // TAIL_MAX clusters
-  int8_t* sm = reinterpret_cast<int8_t*>(sb + 8 * TAIL_MAX);
-  __shared__ uint32_t s_we[32];
-  __shared__ uint32_t s_count, s_insert, s_pass;
+// The state of one tree's last passes in one CTA.
+struct TailState {
+  uint32_t count, insert, pass;
+  uint64_t sum;  // live clusters of the passes run
+};
+
+// Runs every remaining pass of the tree whose live clusters (at most CAP) are
+// cur_g[0, st.count).  `smem`: tail_smem(CAP) bytes.  Returns the shared-memory
+// array that holds the root.
+template <uint32_t CAP, int THREADS>
+__device__ __forceinline__ const float* tail_passes(TailState& t, const Bvh2Node* __restrict__ cur_g, float* smem,
+                                                    uint32_t* s_we, int radius, uint32_t depth_threshold,
+                                                    uint32_t max_passes, Bvh2Node* __restrict__ out, uint32_t* status,
+                                                    const uint32_t* __restrict__ remap, int fast,
+                                                    uint32_t* pass_ins) {
+  float* sa = smem;           // CAP clusters (8 word arrays)
+  float* sb = sa + 8 * CAP;   // CAP clusters
+  int8_t* sm = reinterpret_cast<int8_t*>(sb + 8 * CAP);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    s_pass = st->passes;
-    s_count = st->count[s_pass & 1u];
-    s_insert = st->insert[s_pass & 1u];
-  }
-  __syncthreads();
-  if (s_count > TAIL_MAX) {  // the passes before ended early (their error is set)
-    if (tid == 0) set_status(status, ST_ITER_LIMIT);
-    return;
-  }
-  const int parity = (int)(s_pass & 1u);
-  const Bvh2Node* __restrict__ cur_g = parity ? buf1 : buf0;
-  uint32_t count = s_count;
-  for (uint32_t j = tid; j < count; j += TAIL_THREADS) {
+  uint32_t count = t.count;
+  for (uint32_t j = tid; j < count; j += THREADS) {
     const float4* q = reinterpret_cast<const float4*>(&cur_g[j]);
-    snode_put(sa, j, q[0], q[1]);
+    snode_put<CAP>(sa, j, q[0], q[1]);
   }
   __syncthreads();
   float* cur = sa;
   float* nxt = sb;
-  uint32_t insert = s_insert;
-  uint32_t pass = s_pass;
+  uint32_t insert = t.insert;
+  uint32_t pass = t.pass;
   uint64_t sum = 0;
   uint32_t iters = 0;
   while (count > 1) {
@@ -1395,12 +1390,12 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_ploc_tail(const Bvh2Node* __re
     const int r = d1 ? 1 : radius;
     // search
     if (fast)
-      tail_search<true>(cur, count, d1, r, sm, tid);
+      tail_search<CAP, THREADS, true>(cur, count, d1, r, sm, tid);
     else
-      tail_search<false>(cur, count, d1, r, sm, tid);
+      tail_search<CAP, THREADS, false>(cur, count, d1, r, sm, tid);
     __syncthreads();
     // flags: thread tid owns items [tid*IT, tid*IT + IT)
-    constexpr int IT = TAIL_MAX / TAIL_THREADS;
+    constexpr int IT = (int)CAP / THREADS;
     bool emit[IT], ism[IT];
     uint32_t bst[IT];
     uint32_t e = 0, m = 0;
@@ -1419,7 +1414,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_ploc_tail(const Bvh2Node* __re
       e += emit[k];
       m += ism[k];
     }
-    // (emitted, merged) counts packed in 16 + 16 bits (both at most TAIL_MAX):
+    // (emitted, merged) counts packed in 16 + 16 bits (both at most CAP):
     // a warp scan, then every warp scans the 32 warp totals itself
     uint32_t x = e | (m << 16);
 #pragma unroll
@@ -1429,7 +1424,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_ploc_tail(const Bvh2Node* __re
     }
     if (lane == 31) s_we[warp] = x;
     __syncthreads();
-    uint32_t wt = s_we[lane];
+    uint32_t wt = lane < THREADS / 32 ? s_we[lane] : 0u;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, wt, o);
@@ -1446,8 +1441,8 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_ploc_tail(const Bvh2Node* __re
       if (!emit[k]) continue;
       if (ism[k]) {
         float4 la, lb, ra, rb;
-        snode_get(cur, i, la, lb);
-        snode_get(cur, bst[k], ra, rb);
+        snode_get<CAP>(cur, i, la, lb);
+        snode_get<CAP>(cur, bst[k], ra, rb);
         uint32_t ins = insert - 2 * (mpos + 1);
         if (remap) ins = remap[(ins - 1) >> 1];
         float4* o = reinterpret_cast<float4*>(&out[ins]);
@@ -1457,13 +1452,13 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_ploc_tail(const Bvh2Node* __re
         o[3] = rb;
         Box u = box_union(Box{make_float3(la.x, la.y, la.z), make_float3(lb.x, lb.y, lb.z)},
                           Box{make_float3(ra.x, ra.y, ra.z), make_float3(rb.x, rb.y, rb.z)});
-        snode_put(nxt, epos, make_float4(u.mn.x, u.mn.y, u.mn.z, __uint_as_float(0u)),
+        snode_put<CAP>(nxt, epos, make_float4(u.mn.x, u.mn.y, u.mn.z, __uint_as_float(0u)),
                   make_float4(u.mx.x, u.mx.y, u.mx.z, __uint_as_float(ins)));
         mpos++;
       } else {
         float4 a, b;
-        snode_get(cur, i, a, b);
-        snode_put(nxt, epos, a, b);
+        snode_get<CAP>(cur, i, a, b);
+        snode_put<CAP>(nxt, epos, a, b);
       }
       epos++;
     }
@@ -1471,22 +1466,89 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_ploc_tail(const Bvh2Node* __re
     count = te;
     insert -= 2 * tm;
     pass++;
-    float* t = cur;
+    float* swp = cur;
     cur = nxt;
-    nxt = t;
+    nxt = swp;
     __syncthreads();
   }
+  t = TailState{count, insert, pass, sum};
+  return cur;
+}
+
+constexpr size_t tail_smem(uint32_t cap) { return (size_t)cap * 64 + cap + 64; }
+
+// Finishes every remaining pass (count <= TAIL_MAX) inside one CTA.
+// The live clusters are in buf[passes & 1].
+__global__ void __launch_bounds__(TAIL_THREADS) k_ploc_tail(const Bvh2Node* __restrict__ buf0,
+                                                            const Bvh2Node* __restrict__ buf1, PlocState* st,
+                                                            int radius, uint32_t depth_threshold, uint32_t max_passes,
+                                                            Bvh2Node* __restrict__ out, uint32_t* status,
+                                                            const uint32_t* __restrict__ remap, int fast,
+                                                            uint32_t* pass_ins) {
+  grid_dep_wait();
+  extern __shared__ float4 smem[];
+  __shared__ uint32_t s_we[32];
+  __shared__ uint32_t s_count, s_insert, s_pass;
+  const int tid = threadIdx.x;
   if (tid == 0) {
-    if (pass_ins && pass < PLOC_PASS_REC) pass_ins[pass] = insert;
+    s_pass = st->passes;
+    s_count = st->count[s_pass & 1u];
+    s_insert = st->insert[s_pass & 1u];
+  }
+  __syncthreads();
+  if (s_count > TAIL_MAX) {  // the passes before ended early (their error is set)
+    if (tid == 0) set_status(status, ST_ITER_LIMIT);
+    return;
+  }
+  const int parity = (int)(s_pass & 1u);
+  TailState t{s_count, s_insert, s_pass, 0};
+  const float* cur = tail_passes<TAIL_MAX, TAIL_THREADS>(t, parity ? buf1 : buf0, reinterpret_cast<float*>(smem), s_we,
+                                                         radius, depth_threshold, max_passes, out, status, remap, fast,
+                                                         pass_ins);
+  if (tid == 0) {
+    if (pass_ins && t.pass < PLOC_PASS_REC) pass_ins[t.pass] = t.insert;
     float4* o = reinterpret_cast<float4*>(&out[0]);
-    snode_get(cur, 0, o[0], o[1]);
-    st->count[parity] = count;
-    st->insert[parity] = insert;
-    st->passes = pass;
-    st->sum_counts += sum;
+    snode_get<TAIL_MAX>(cur, 0, o[0], o[1]);
+    st->count[parity] = t.count;
+    st->insert[parity] = t.insert;
+    st->passes = t.pass;
+    st->sum_counts += t.sum;
   }
 }
 
+// The last passes of every scene of a segmented build, a CTA per scene: from
+// the pass at which k_ploc_seg left it (count at most SEG_TAIL_MAX) to the root.
+// A scene's late passes are latency, not work: in k_ploc_seg each of them costs
+// the whole batch two grid barriers, here block barriers beside the other
+// scenes'.  Batches of 96 scenes of 1k-200k triangles 7194 -> 6558 us, 20 of
+// 2k-50k 2475 -> 2072, 40 of 1k-3k 1547 -> 1239, 512 of 1k-60k 25.03 -> 24.33
+// ms.  Leaving scenes to it at 1,024 clusters instead of 2,048: 6629 / 2102 /
+// 1268 us / 24.35 ms; at 512: 6698 / 2157 / 1303 / 24.37.
+__global__ void __launch_bounds__(SEG_TAIL_THREADS) k_ploc_seg_tail(PlocSegArgs a) {
+  grid_dep_wait();
+  extern __shared__ float4 smem[];
+  __shared__ uint32_t s_we[32];
+  const uint32_t s = blockIdx.x;
+  const int tid = threadIdx.x;
+  const uint32_t pass = a.passes[s];
+  const size_t at = (size_t)(pass & 1u) * a.n_seg + s;
+  const uint32_t count = a.count[at], cb = a.prim_start[s], nb = a.node_start[s];
+  if (count <= 1) return;      // no leaves, one leaf (k_ploc_seg_init wrote the root) or a failed scene
+  if (count > SEG_TAIL_MAX) {  // the passes before ended early (their error is set)
+    if (tid == 0) set_status(a.status, ST_ITER_LIMIT);
+    return;
+  }
+  TailState t{count, a.insert[at], pass, 0};
+  const float* cur = tail_passes<SEG_TAIL_MAX, SEG_TAIL_THREADS>(
+      t, ((pass & 1u) ? a.buf[1] : a.buf[0]) + cb, reinterpret_cast<float*>(smem), s_we, a.radius, a.depth_threshold,
+      a.max_passes, a.out, a.status, nullptr, 1, nullptr);
+  if (tid == 0) {
+    float4* o = reinterpret_cast<float4*>(&a.out[nb]);
+    snode_get<SEG_TAIL_MAX>(cur, 0, o[0], o[1]);
+    a.passes[s] = t.pass;
+    a.sum_counts[s] += t.sum;
+  }
+}
 
 // --- the last passes on one thread-block cluster ------------------------------
 //
@@ -2134,8 +2196,7 @@ int ploc_build_device(BuildCtx& c, Bvh2Node* leaves, uint32_t n, const int* tota
     KLAUNCH("k_ploc_cluster", CK(cudaLaunchKernelEx(&cfg, k_ploc_cluster, ca)));
   }
   {
-    const size_t smem = (size_t)4 * TAIL_MAX * sizeof(float4) + TAIL_MAX + 64;
-    KLAUNCH("k_ploc_tail", launch_k(k_ploc_tail, 1, TAIL_THREADS, smem, c.stream, cur, nxt, st, (int)radius, depth_threshold,
+    KLAUNCH("k_ploc_tail", launch_k(k_ploc_tail, 1, TAIL_THREADS, tail_smem(TAIL_MAX), c.stream, cur, nxt, st, (int)radius, depth_threshold,
                                                                            max_passes, out_nodes, c.d_status, remap,
                                     nan_checked ? 1 : 0, pass_ins));
     CK(cudaGetLastError());
@@ -2229,12 +2290,18 @@ int ploc_seg_device(BuildCtx& c, const SegLayout& L, const Bvh2Node* leaves, con
   PlocSegArgs pa{{cur, nxt}, out, merge, tile_cnt, L.d_prim_start, L.d_node_start, count, insert, d_passes,
                  d_sum_counts, ctl, S, (int)radius, depth_threshold, 2 * L.max_m + 64, c.d_status};
   void* args[] = {&pa};
-  KLAUNCH("k_ploc_seg", CK(coop_launch(c, (const void*)k_ploc_seg, seg_blocks, COOP_GROUPS * PT, args, smem)));
+  if (L.max_m > SEG_TAIL_MAX)
+    KLAUNCH("k_ploc_seg", CK(coop_launch(c, (const void*)k_ploc_seg, seg_blocks, COOP_GROUPS * PT, args, smem)));
+  KLAUNCH("k_ploc_seg_tail", launch_k(k_ploc_seg_tail, S, SEG_TAIL_THREADS, tail_smem(SEG_TAIL_MAX), c.stream, pa));
+  CK(cudaGetLastError());
   return 0;
 }
 
 int ploc_setup_kernels() {
-  size_t smem = (size_t)4 * TAIL_MAX * sizeof(float4) + TAIL_MAX + 64;
-  cudaError_t e = cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return e == cudaSuccess ? 0 : -1;
+  return cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tail_smem(TAIL_MAX)) ==
+                     cudaSuccess &&
+                 cudaFuncSetAttribute(k_ploc_seg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)tail_smem(SEG_TAIL_MAX)) == cudaSuccess
+             ? 0
+             : -1;
 }
