@@ -32,8 +32,9 @@ def _is_cuda_tensor(x) -> bool:
     return hasattr(x, "is_cuda") and hasattr(x, "data_ptr") and bool(x.is_cuda)
 
 
-def _prep(x, dtype, cols):
-    """Returns (pointer, n_rows, device_flag, keepalive)."""
+def _prep(x, dtype, cols, wait=True):
+    """Returns (pointer, n_rows, device_flag, keepalive).  Without `wait` the
+    caller waits for the tensors' producers itself (_prep_many)."""
     if _is_cuda_tensor(x):
         import torch
 
@@ -43,13 +44,27 @@ def _prep(x, dtype, cols):
         x = x.contiguous()
         # the tensor's producer ran on torch's current stream; the library's
         # work goes on its own stream
-        torch.cuda.current_stream(x.device).synchronize()
+        if wait:
+            torch.cuda.current_stream(x.device).synchronize()
         n = x.numel() // cols if cols else x.numel()
         return ctypes.c_void_p(x.data_ptr()), n, 1, x
     a = np.ascontiguousarray(x, dtype=dtype)
     if cols:
         a = a.reshape(-1, cols)
     return a.ctypes.data_as(ctypes.c_void_p), (len(a) if cols else a.size), 0, a
+
+
+def _prep_many(xs, dtype, cols):
+    """_prep of several arrays, waiting once per device instead of once per
+    array (96 scenes: 0.4 ms of host time)."""
+    preps = [_prep(x, dtype, cols, wait=False) for x in xs]
+    devices = {p[3].device for p in preps if p[2]}
+    if devices:
+        import torch
+
+        for d in devices:
+            torch.cuda.current_stream(d).synchronize()
+    return preps
 
 
 class Context:
@@ -604,7 +619,7 @@ def build_cwbvh_from_tris_segmented(scenes, config: BvhBuildParams, ctx: Context
     CWBVH launches that cover every scene).  Each result is byte-identical to
     building that scene alone; the results share one device allocation."""
     ctx = _ctx(ctx)
-    preps = [_prep(t, np.float32, 9) for t in scenes]
+    preps = _prep_many(scenes, np.float32, 9)
     devs = {p[2] for p in preps}
     if len(devs) > 1:
         raise ValueError("scenes must all be host arrays or all device tensors")
@@ -635,7 +650,7 @@ def build_cwbvh_from_tris_batch(scenes, config: BvhBuildParams, contexts=None) -
     if not contexts:
         raise ValueError("at least one context")
     ctx = contexts[0]
-    preps = [_prep(t, np.float32, 9) for t in scenes]
+    preps = _prep_many(scenes, np.float32, 9)
     devs = {p[2] for p in preps}
     if len(devs) > 1:
         raise ValueError("scenes must all be host arrays or all device tensors")
@@ -712,9 +727,14 @@ def ray_traverse_batches(bvhs, batch_bvh, rays, outs=None, ctx: Context | None =
     return outs
 
 
+#: ids a query call has room for at first: per query, and at most
+QUERY_IDS_EACH, QUERY_IDS_MOST = 32, 1 << 20
+
+
 def _query(obj, fn, kind, queries, prim_aabbs, extra):
-    """Two calls of an obvhs_*_query entry (sizes, then ids): a list of uint32
-    arrays of original primitive ids, one per query."""
+    """A call of an obvhs_*_query entry with room for a guessed number of ids,
+    and a second one when there are more: a list of uint32 arrays of original
+    primitive ids, one per query."""
     k = 0 if kind == "aabb" else 1
     q = np.ascontiguousarray(queries, dtype=np.float32).reshape(-1, 6 if k == 0 else 3)
     pa = None if prim_aabbs is None else np.ascontiguousarray(prim_aabbs, dtype=np.float32).reshape(-1, 6)
@@ -722,10 +742,14 @@ def _query(obj, fn, kind, queries, prim_aabbs, extra):
     off = np.zeros(n + 1, np.uint32)
     args = [obj.ctx.h, obj.h, k, q.ctypes.data_as(ctypes.c_void_p), n,
             None if pa is None else pa.ctypes.data_as(ctypes.c_void_p), 0 if pa is None else len(pa)] + extra
-    obj.ctx.check(fn(*args, off.ctypes.data_as(ctypes.c_void_p), None, 0, 0))
-    ids = np.zeros(max(int(off[n]), 1), np.uint32)
-    obj.ctx.check(fn(*args, off.ctypes.data_as(ctypes.c_void_p), ids.ctypes.data_as(ctypes.c_void_p), len(ids), 0))
-    return [ids[int(off[i]):int(off[i + 1])].copy() for i in range(n)]
+    ids = np.zeros(min(QUERY_IDS_EACH * n + 1024, QUERY_IDS_MOST), np.uint32)
+    for _ in range(2):
+        obj.ctx.check(fn(*args, off.ctypes.data_as(ctypes.c_void_p), ids.ctypes.data_as(ctypes.c_void_p), len(ids), 0))
+        if int(off[n]) <= len(ids):
+            break
+        ids = np.zeros(int(off[n]), np.uint32)
+    o = off.tolist()
+    return [ids[a:b].copy() for a, b in zip(o, o[1:])]
 
 
 def _params(p: BvhBuildParams) -> N.BuildParams:
