@@ -8,7 +8,7 @@
 //
 // Costs: a parent-counter climb from the leaves (the second child to arrive
 // computes the parent, carrying its own child's record in registers and
-// reading only the sibling's).  Besides the 7 decisions, every node records
+// reading only the sibling's; small trees with eight lanes a node).  Besides the 7 decisions, every node records
 // for each slot budget j the number of CWBVH nodes it contributes when its
 // parent's distribution reaches it with budget j, so the count below the
 // children of any decision is one add and no record needs a tree walk; the
@@ -528,6 +528,195 @@ __global__ void __launch_bounds__(BLK) k_costs(const Bvh2Node* __restrict__ node
   }
 }
 
+constexpr uint32_t FULL_MASK = 0xffffffffu;
+
+// Octet-wide operations (width-8 shuffles: all 32 lanes take part, each
+// octet reduces its own lanes).
+__device__ __forceinline__ uint32_t oct_excl_scan(uint32_t v, int sub, uint32_t* total) {
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL_MASK, x, o, 8);
+    if (sub >= o) x += y;
+  }
+  *total = __shfl_sync(FULL_MASK, x, 7, 8);
+  return x - v;
+}
+__device__ __forceinline__ uint32_t oct_bits(uint32_t ballot, int lane) { return (ballot >> (lane & 24)) & 0xffu; }
+
+// The climb with eight lanes (an octet) per node, for trees too small to fill
+// the GPU, whose time is the chain of levels from the deepest leaf: lane i
+// holds slot i of the record (lane 7 the decisions and the primitive count), so
+// a level's 28 candidate sums are a shuffle chain of about 100 instructions
+// instead of 330 dependent ones in one thread, and a record is two coalesced
+// 32-byte accesses.  Same records, same arithmetic per slot, as inner_rec.
+// 4k nodes after reinsertion 95 -> 33 us, 20k nodes from PLOC (ready flags
+// polled level by level before) 120 -> 41 us.
+__global__ void __launch_bounds__(BLK) k_costs_oct(const Bvh2Node* __restrict__ nodes, const uint32_t* __restrict__ parents,
+                                                   const uint32_t* __restrict__ pidx_in, uint32_t n, uint32_t max_prims,
+                                                   CostRec* crec, EmitRec* erec, uint4* small, uint32_t* flags,
+                                                   uint32_t* status) {
+  grid_dep_wait();
+  const float INF = __int_as_float(0x7f800000);
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  const uint32_t n_oct = gridDim.x * (BLK / 8);
+  uint32_t next = (blockIdx.x * BLK + threadIdx.x) >> 3;  // this octet's next leaf candidate
+  uint32_t c = 0, p = 0, nprim = 0, meta = 0, contrib = 0, steps = 0;
+  float cost = 0.0f;
+  uint4 list = make_uint4(0u, 0u, 0u, 0u);
+  bool climbing = false, leaf = false;
+  for (;;) {
+    // a new climb for every octet without one
+    while (!climbing && next < n) {
+      const uint32_t i = next;
+      next += n_oct;
+      const Bvh2Node nd = ld_node(&nodes[i]);
+      if (node_prims(nd) == 0) continue;
+      if (node_prims(nd) != 1) {  // src/cwbvh/bvh2_to_cwbvh.rs:243-247
+        if (sub == 0) set_status(status, ST_BAD_INPUT);
+        continue;
+      }
+      list = make_uint4(__ldg(&pidx_in[node_first(nd)]), 0u, 0u, 1u);
+      p = parents[i];
+      if (sub == 0) {
+        __stcg(&small[i], list);
+        if (p == i) __stcg(&erec[i], make_uint4(0u, 0u, 1u, 0u));  // a leaf root: one CWBVH node
+      }
+      if (p == i) continue;
+      const CostRec r = leaf_rec(nd);
+      cost = r.cost[0];
+      contrib = 0;
+      meta = 0;
+      nprim = 1;
+      leaf = climbing = true;
+      c = i;
+      steps = 0;
+    }
+    if (__ballot_sync(FULL_MASK, climbing) == 0) {
+      if (__ballot_sync(FULL_MASK, next < n) == 0) return;
+      continue;
+    }
+    // one level, as CostClimb::step
+    Bvh2Node pn{}, sg_node{};
+    uint32_t up = 0, sg = 0;
+    if (climbing) {
+      if (++steps > n) {
+        if (sub == 0) set_status(status, ST_ITER_LIMIT);
+        climbing = false;
+      } else {
+        pn = ld_node(&nodes[p]);
+        up = parents[p];
+        sg = sibling_of(c);
+        if (sg >= n) sg = c;  // a tree that breaks the rule: the real sibling is read below
+        sg_node = ld_node(&nodes[sg]);
+        if (!leaf) {
+          uint32_t* w = reinterpret_cast<uint32_t*>(&crec[c]);
+          __stcg(w + sub, sub == 7 ? meta : __float_as_uint(cost));
+          __stcg(w + 8 + sub, sub == 7 ? nprim : contrib);
+        }
+      }
+    }
+    __syncwarp();
+    uint32_t first = 0;
+    if (climbing && sub == 0) first = atom_add_acq_rel(&flags[p], 1u) == 0 ? 1u : 0u;
+    first = __shfl_sync(FULL_MASK, first, 0, 8);
+    if (first) climbing = false;  // the sibling's climb continues
+    const uint32_t f = node_first(pn);
+    const bool own_left = c == f;
+    float oc = 0.0f;
+    uint32_t ocn = 0, onp = 0;
+    uint4 ol = make_uint4(0u, 0u, 0u, 0u);
+    if (climbing) {
+      const uint32_t s = own_left ? f + 1 : f;
+      const Bvh2Node sn = s == sg ? sg_node : ld_node(&nodes[s]);
+      if (node_prims(sn) != 0) {
+        oc = leaf_rec(sn).cost[0];
+        onp = 1;
+        ol = make_uint4(__ldg(&pidx_in[node_first(sn)]), 0u, 0u, 1u);
+      } else {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(&crec[s]);
+        oc = __uint_as_float(__ldcg(w + sub));  // (lane 7: the decisions, not read)
+        ocn = __ldcg(w + 8 + sub);
+        onp = __ldcg(w + 15);
+        if (nprim + onp <= 3) ol = __ldcg(&small[s]);
+      }
+    }
+    // calculate_cost_impl (src/cwbvh/bvh2_to_cwbvh.rs:257-341), slot by lane
+    const float L = own_left ? cost : oc, R = own_left ? oc : cost;
+    const uint32_t Lc = own_left ? contrib : ocn, Rc = own_left ? ocn : contrib;
+    const uint32_t np = nprim + onp;
+    const float ha = half_area(node_box(pn));
+    // slot 0: the best of L[k] + R[6 - k], candidate k in lane k, the first on ties
+    float best = L + __shfl_sync(FULL_MASK, R, 6 - min(sub, 6), 8);
+    uint32_t bk = (uint32_t)sub;
+    if (sub == 7 || !(best < INF)) {
+      best = INF;
+      bk = DL_INVALID;
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(FULL_MASK, best, o, 8);
+      const uint32_t okk = __shfl_xor_sync(FULL_MASK, bk, o, 8);
+      if (ob < best || (ob == best && okk < bk)) {
+        best = ob;
+        bk = okk;
+      }
+    }
+    uint32_t agg0 = add_agg(__shfl_sync(FULL_MASK, Lc, (int)min(bk, 6u), 8),
+                            __shfl_sync(FULL_MASK, Rc, 6 - (int)min(bk, 6u), 8));
+    if (bk == DL_INVALID) agg0 = AGG_INVALID;
+    const float cost_leaf = np <= max_prims ? ((float)np * ha) * PRIM_COST : INF;
+    const float ci = best + ha;
+    const bool internal = !(cost_leaf < ci);
+    const uint32_t contrib0 = internal ? (agg0 == AGG_INVALID ? AGG_INVALID : 1u + agg0) : 0u;
+    // slot i > 0: the best of L[k] + R[i - 1 - k], k < i, the first on ties
+    float d = INF;
+    uint32_t dl = 0;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      const float x = __shfl_sync(FULL_MASK, L, k, 8) + __shfl_sync(FULL_MASK, R, max(sub - 1 - k, 0), 8);
+      if (k < sub && sub < 7 && x < d) {
+        d = x;
+        dl = (uint32_t)k;
+      }
+    }
+    const uint32_t la = __shfl_sync(FULL_MASK, Lc, (int)dl, 8);
+    const uint32_t ra = __shfl_sync(FULL_MASK, Rc, max(sub - 1 - (int)dl, 0), 8);
+    // cost[i] = d_i where that is below cost[i - 1], else cost[i - 1]
+    float x = sub == 0 ? (internal ? ci : cost_leaf) : d;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const float y = __shfl_up_sync(FULL_MASK, x, o, 8);
+      if (sub >= o && !(x < y)) x = y;
+    }
+    const float prev = __shfl_up_sync(FULL_MASK, x, 1, 8);
+    const bool dist = sub > 0 && sub < 7 && d < prev;
+    const uint32_t dmask = oct_bits(__ballot_sync(FULL_MASK, dist), lane) & ((2u << sub) - 1u);
+    const uint32_t agg_own = add_agg(la, ra);
+    const uint32_t agg_at = __shfl_sync(FULL_MASK, agg_own, dmask ? 31 - __clz(dmask) : 0, 8);
+    uint32_t m = sub == 0 ? ((internal ? 8u : 0u) | bk) : dist ? (8u | dl) << (4 * sub) : 0u;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) m |= __shfl_xor_sync(FULL_MASK, m, o, 8);
+    if (climbing) {
+      if (np <= 3) {
+        list = concat_lists(own_left ? list : ol, own_left ? ol : list);
+        if (sub == 1) __stcg(&small[p], list);
+      } else {
+        list = make_uint4(0u, 0u, 0u, np);
+      }
+      if (sub == 0) __stcg(&erec[p], make_uint4(m, agg0, np, 0u));
+      cost = x;
+      contrib = dmask ? agg_at : contrib0;
+      meta = m;
+      nprim = np;
+      leaf = false;
+      climbing = up != p;
+      c = p;
+      p = up;
+    }
+  }
+}
+
 __device__ __forceinline__ float pow2f(float c) {
   if (c >= 128.0f) return __int_as_float(0x7f800000);
   if (c >= -126.0f) return __int_as_float(((int)c + 127) << 23);
@@ -591,22 +780,6 @@ struct EmitArgs {
 // one entry per lane, each child's records are loaded by its own lane, the
 // greedy slot assignment reduces over the octet with shuffles, and each lane
 // publishes, quantises and writes its own child.
-constexpr uint32_t FULL_MASK = 0xffffffffu;
-
-// Octet-wide operations (width-8 shuffles: all 32 lanes take part, each
-// octet reduces its own lanes).
-__device__ __forceinline__ uint32_t oct_excl_scan(uint32_t v, int sub, uint32_t* total) {
-  uint32_t x = v;
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(FULL_MASK, x, o, 8);
-    if (sub >= o) x += y;
-  }
-  *total = __shfl_sync(FULL_MASK, x, 7, 8);
-  return x - v;
-}
-__device__ __forceinline__ uint32_t oct_bits(uint32_t ballot, int lane) { return (ballot >> (lane & 24)) & 0xffu; }
-
 struct OctetShared {
   uint2 list[8];           // distribution walk entries
   uint8_t slot_child[8];   // child placed in each slot (0xff: empty)
@@ -1296,6 +1469,28 @@ static uint32_t cost_grid(BuildCtx& c, uint32_t n) {
   return (uint32_t)std::min<uint64_t>((uint64_t)per_sm * c.num_sms, std::max<uint32_t>(1, div_up<uint32_t>(n, BLK)));
 }
 
+// Trees of at most this many BVH2 nodes are costed eight lanes a node.  Below
+// it the levels' latency counts (builds of 10k triangles from PLOC 637 -> 553
+// us, 30k 589 -> 511, 2k after reinsertion 512 -> 482; 30k after reinsertion
+// even); above it the octets' throughput does: 200k nodes after reinsertion 75
+// us a thread per node, 191 an octet, 200k from PLOC even, 600k 1092 against
+// 1302 us for the build.
+constexpr uint32_t COST_OCT_MAX = 65536;
+
+// Blocks of k_costs_oct: an octet per node, or every resident slot.
+static uint32_t cost_oct_grid(BuildCtx& c, uint32_t n) {
+  static std::atomic<int> per_sm_s{0};
+  int per_sm = per_sm_s.load();
+  if (!per_sm) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_costs_oct, BLK, 0) != cudaSuccess || per_sm < 1) {
+      cudaGetLastError();
+      per_sm = 1;
+    }
+    per_sm_s.store(per_sm);
+  }
+  return (uint32_t)std::min<uint64_t>((uint64_t)per_sm * c.num_sms, std::max<uint32_t>(1, div_up<uint32_t>(n, BLK / 8)));
+}
+
 // Blocks of the cooperative range-ordered cost pass: every resident slot.
 static uint32_t cost_range_grid(BuildCtx& c) {
   static std::atomic<int> per_sm_s{0};
@@ -1353,7 +1548,13 @@ int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, i
   // the tree came straight from this context's last PLOC build: cost it
   // range by range (a cooperative launch), unless the GPU is shared
   const bool ranges = ploc_passes > 0 && ploc_passes < PLOC_PASS_REC && c.ploc_pass_ins && !gpu_shared(c);
-  if (ranges) {  // (the kernel clears the flags it uses)
+  if (n <= COST_OCT_MAX) {
+    CK(cudaMemsetAsync(flags, 0, (size_t)n * 4 + 8, c.stream));
+    int r = compute_parents_device(c, b->nodes, n, parents);
+    if (r) return r;
+    KLAUNCH("k_costs_oct", launch_k(k_costs_oct, cost_oct_grid(c, n), BLK, 0, c.stream, b->nodes, parents, b->prim_indices,
+                                    n, max_prims, crec, erec, small, flags, c.d_status));
+  } else if (ranges) {  // (the kernel clears the flags it uses)
     CostRangeArgs ra{b->nodes, b->prim_indices, c.ploc_pass_ins, n, max_prims, ploc_passes, crec, erec, small,
                      c.d_status};
     uint32_t* fl = flags;
