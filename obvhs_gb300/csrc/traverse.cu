@@ -315,9 +315,12 @@ __device__ __forceinline__ void persistent_rays(R& ray, uint32_t nrays, uint32_t
 // 13.47 / 1615 / 1556.
 constexpr int VOTED_REFILL_IDLE = 6;
 template <class R, int TB = TBLK>
-__device__ __forceinline__ void voted_rays(R& ray, uint32_t nrays, uint32_t* next_ray, const uint32_t* yield) {
+__device__ __forceinline__ void voted_rays(R& ray, uint32_t nrays, uint32_t* next_ray, const uint32_t* yield,
+                                           uint32_t lanes = 32) {
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  const bool takes = (uint32_t)lane < lanes;  // this lane may hold a ray
+  const int refill_at = (int)lanes - (lanes == 32 ? VOTED_REFILL_IDLE : 1);
   const uint32_t lt_mask = (1u << lane) - 1u;
   bool alive = false;    // this lane holds a ray
   bool drained = false;  // (warp-uniform) the ray counter has run out
@@ -333,14 +336,14 @@ __device__ __forceinline__ void voted_rays(R& ray, uint32_t nrays, uint32_t* nex
       if (__shfl_sync(FULL, y, 0)) drained = true;
     }
     if (!drained) {
-      const uint32_t need = __ballot_sync(FULL, !alive);
+      const uint32_t need = __ballot_sync(FULL, takes && !alive);
       if (need) {
         const int leader = __ffs(need) - 1;
         uint32_t base = 0;
         if (lane == leader) base = atomicAdd(next_ray, (uint32_t)__popc(need));
         base = __shfl_sync(FULL, base, leader);
         if ((uint64_t)base + __popc(need) >= nrays) drained = true;
-        if (!alive) {
+        if (takes && !alive) {
           const uint32_t ri = base + __popc(need & lt_mask);
           if (ri < nrays) alive = ray.start(ri);
         }
@@ -353,7 +356,7 @@ __device__ __forceinline__ void voted_rays(R& ray, uint32_t nrays, uint32_t* nex
     for (;;) {
       const bool want_prim = alive && ray.has_prim();
       const uint32_t mp = __ballot_sync(FULL, want_prim), ma = __ballot_sync(FULL, alive);
-      if (ma == 0 || (!drained && __popc(ma) <= 32 - VOTED_REFILL_IDLE)) break;
+      if (ma == 0 || (!drained && __popc(ma) <= refill_at)) break;
       if (4 * __popc(mp) >= __popc(ma & ~mp)) {
         if (want_prim && ray.prim_step()) alive = false;
       } else {
@@ -522,7 +525,7 @@ struct CwRay {
 // per thread, entry k of thread t at [k][t]: consecutive threads' entries
 // are adjacent, so a warp's pushes and pops are conflict-free) instead of
 // the thread's local memory.  Same loop, same results.
-template <int MODE, bool CTRI = false, bool MULTI = false, int TB = TBLK, bool SST = false>
+template <int MODE, bool CTRI = false, bool MULTI = false, int TB = TBLK, bool SST = false, bool FEW = false>
 __global__ void __launch_bounds__(TB) k_traverse(const CwNode* __restrict__ nodes_in, uint32_t n_nodes_in,
                                                    const float4* __restrict__ tris_in, uint32_t n_prims_in,
                                                    const float4* __restrict__ rays,
@@ -532,7 +535,7 @@ __global__ void __launch_bounds__(TB) k_traverse(const CwNode* __restrict__ node
                                                    const uint32_t* __restrict__ pidx = nullptr,
                                                    const BlasDesc* __restrict__ multi = nullptr,
                                                    const uint32_t* __restrict__ ray_bvh = nullptr, uint32_t n_multi = 0,
-                                                   const uint32_t* yield = nullptr) {
+                                                   const uint32_t* yield = nullptr, uint32_t lanes = 32) {
   grid_dep_wait();
   uint2 lstack[SST ? 1 : 32];
   __shared__ uint2 sstack[SST ? 32 * TB : 1];
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(TB) k_traverse(const CwNode* __restrict__ node
   ray.multi = multi;
   ray.ray_bvh = ray_bvh;
   ray.n_multi = n_multi;
-  voted_rays<decltype(ray), TB>(ray, nrays, next_ray, yield);
+  voted_rays<decltype(ray), TB>(ray, nrays, next_ray, yield, FEW ? lanes : 32u);
 }
 
 // The traversal launch forms a context can choose (obvhs_ctx_set_traversal_config):
@@ -563,16 +566,30 @@ struct TravForm {
 constexpr TravForm TRAV_FORMS[] = {{128, false}, {64, false}, {256, false}, {64, true}, {128, true}};
 constexpr int N_TRAV_FORMS = 5;
 
+// Rays a warp takes at a time.  A call of few rays is a chain of dependent
+// loads per ray, and a warp takes the time of all its rays' different steps
+// together, so they are spread: one ray a warp while that gives each of the
+// SMs' four schedulers at most two warps, then two, four, ... (1,000 host rays
+// on 10k triangles 88.6 -> 78.9 us the call, 3,000 on 100k 111.6 -> 105.2,
+// 14,400 149 -> 144; from 30,000 rays even.  Four warps a scheduler: 30,000
+// rays 159 -> 167 us; one: 3,000 rays 108 us).  The kernels that take 32 are
+// compiled apart: with the count in a register they ran 1-1.6 % slower.
+inline uint32_t rays_per_warp(const BuildCtx& c, uint32_t n) {
+  uint32_t lanes = 1;
+  while (lanes < 32 && (uint64_t)lanes * c.num_sms * 8 < n) lanes *= 2;
+  return lanes;
+}
+
 // Launches k_traverse<MODE, false, MULTI> in form f as a persistent grid
 // (resident blocks, or fewer for a small batch).
-template <int MODE, bool MULTI, int TB, bool SST>
+template <int MODE, bool MULTI, int TB, bool SST, bool FEW = false>
 cudaError_t launch_trav_form(BuildCtx& c, uint32_t n, const CwNode* nodes, uint32_t n_nodes, const float4* tris,
                              uint32_t n_prims, const float4* rays, uint2* hits, uint8_t* miss, uint32_t* counter,
-                             const BlasDesc* dd, const uint32_t* ray_bvh, uint32_t n_bvh) {
+                             const BlasDesc* dd, const uint32_t* ray_bvh, uint32_t n_bvh, uint32_t lanes = 32) {
   static std::atomic<int> per_sm_s{0};
   int per_sm = per_sm_s.load();
   if (!per_sm) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_traverse<MODE, false, MULTI, TB, SST>, TB, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_traverse<MODE, false, MULTI, TB, SST, FEW>, TB, 0) !=
             cudaSuccess ||
         per_sm < 1) {
       cudaGetLastError();
@@ -580,13 +597,13 @@ cudaError_t launch_trav_form(BuildCtx& c, uint32_t n, const CwNode* nodes, uint3
     }
     per_sm_s.store(per_sm);
   }
-  const uint32_t grid = std::min<uint32_t>(div_up<uint32_t>(n, TB), (uint32_t)(per_sm * c.num_sms));
+  const uint32_t grid = std::min<uint32_t>(div_up<uint32_t>(n, TB / 32 * lanes), (uint32_t)(per_sm * c.num_sms));
   const char* name = MULTI ? (MODE == 0 ? "k_traverse_closest_multi" : "k_traverse_occluded_multi")
                            : (MODE == 0 ? "k_traverse_closest" : "k_traverse_occluded");
   c.kbegin(name);
-  launch_k(k_traverse<MODE, false, MULTI, TB, SST>, grid, TB, 0, c.stream, nodes, n_nodes, tris, n_prims, rays, n,
+  launch_k(k_traverse<MODE, false, MULTI, TB, SST, FEW>, grid, TB, 0, c.stream, nodes, n_nodes, tris, n_prims, rays, n,
            hits, miss, counter, c.d_status, (const uint2*)nullptr, (const uint32_t*)nullptr, dd, ray_bvh, n_bvh,
-           c.d_yield);
+           c.d_yield, lanes);
   c.kend();
   return cudaGetLastError();
 }
@@ -595,6 +612,10 @@ template <int MODE, bool MULTI>
 cudaError_t launch_trav(BuildCtx& c, uint32_t n, const CwNode* nodes, uint32_t n_nodes, const float4* tris,
                         uint32_t n_prims, const float4* rays, uint2* hits, uint8_t* miss, uint32_t* counter,
                         const BlasDesc* dd, const uint32_t* ray_bvh, uint32_t n_bvh) {
+  const uint32_t lanes = rays_per_warp(c, n);
+  if (lanes < 32)
+    return launch_trav_form<MODE, MULTI, TBLK, false, true>(c, n, nodes, n_nodes, tris, n_prims, rays, hits, miss, counter,
+                                                            dd, ray_bvh, n_bvh, lanes);
   switch (c.trav_form) {
     case 1:
       return launch_trav_form<MODE, MULTI, 64, false>(c, n, nodes, n_nodes, tris, n_prims, rays, hits, miss, counter,
@@ -1359,6 +1380,30 @@ int compress_tris_device(BuildCtx& c, obvhs_cwbvh* b, const float* tris, uint32_
   return 0;
 }
 
+// k_traverse on the compressed triangles, as launch_trav_form.
+template <int MODE, bool FEW>
+static cudaError_t launch_ctri(BuildCtx& c, const obvhs_cwbvh* bvh, const float* rays, uint32_t n, uint32_t* hits,
+                               uint8_t* miss, uint32_t* counter, uint32_t lanes) {
+  static std::atomic<int> per_sm_s{0};
+  int per_sm = per_sm_s.load();
+  if (!per_sm) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_traverse<MODE, true, false, TBLK, false, FEW>, TBLK,
+                                                      0) != cudaSuccess ||
+        per_sm < 1) {
+      cudaGetLastError();
+      per_sm = 1;
+    }
+    per_sm_s.store(per_sm);
+  }
+  const uint32_t grid = std::min<uint32_t>(div_up<uint32_t>(n, TBLK / 32 * lanes), (uint32_t)(per_sm * c.num_sms));
+  c.kbegin(MODE == 0 ? "k_traverse_closest_ctri" : "k_traverse_occluded_ctri");
+  launch_k(k_traverse<MODE, true, false, TBLK, false, FEW>, grid, TBLK, 0, c.stream, bvh->nodes, bvh->n_nodes,
+           (const float4*)nullptr, bvh->n_prims, (const float4*)rays, n, (uint2*)hits, miss, counter, c.d_status,
+           bvh->ctris, bvh->prim_indices, (const BlasDesc*)nullptr, (const uint32_t*)nullptr, 0u, c.d_yield, lanes);
+  c.kend();
+  return cudaGetLastError();
+}
+
 int traverse_compressed_device(BuildCtx& c, const obvhs_cwbvh* bvh, const float* rays, uint32_t n, uint32_t* hits,
                                uint8_t* miss, int mode) {
   if (n == 0) return 0;
@@ -1366,27 +1411,13 @@ int traverse_compressed_device(BuildCtx& c, const obvhs_cwbvh* bvh, const float*
   uint32_t* counter = (uint32_t*)c.scratch.get(SLOT_OUTPUT, 16);
   if (!counter) return c.fail(OBVHS_ERR_OOM, "scratch");
   CK(cudaMemsetAsync(counter, 0, 4, c.stream));
-  static std::atomic<int> per_sm_s{0};
-  int per_sm = per_sm_s.load();
-  if (!per_sm) {
-    int a = 0, b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_traverse<0, true>, TBLK, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_traverse<1, true>, TBLK, 0);
-    per_sm = std::max(1, std::min(a, b));
-    per_sm_s.store(per_sm);
-  }
-  const uint32_t grid = std::min<uint32_t>(div_up<uint32_t>(n, TBLK), (uint32_t)(per_sm * c.num_sms));
-  if (mode == 0)
-    KLAUNCH("k_traverse_closest_ctri", launch_k(k_traverse<0, true>, grid, TBLK, 0, c.stream,
-                                           bvh->nodes, bvh->n_nodes, nullptr, bvh->n_prims, (const float4*)rays, n,
-                                           (uint2*)hits, nullptr, counter, c.d_status, bvh->ctris, bvh->prim_indices, nullptr, nullptr, 0u,
-                                           c.d_yield));
+  const uint32_t lanes = rays_per_warp(c, n);
+  if (lanes < 32)
+    CK((mode == 0 ? launch_ctri<0, true>(c, bvh, rays, n, hits, miss, counter, lanes)
+                  : launch_ctri<1, true>(c, bvh, rays, n, hits, miss, counter, lanes)));
   else
-    KLAUNCH("k_traverse_occluded_ctri", launch_k(k_traverse<1, true>, grid, TBLK, 0, c.stream,
-                                            bvh->nodes, bvh->n_nodes, nullptr, bvh->n_prims, (const float4*)rays, n,
-                                            nullptr, miss, counter, c.d_status, bvh->ctris, bvh->prim_indices, nullptr, nullptr, 0u,
-                                            c.d_yield));
-  CK(cudaGetLastError());
+    CK((mode == 0 ? launch_ctri<0, false>(c, bvh, rays, n, hits, miss, counter, lanes)
+                  : launch_ctri<1, false>(c, bvh, rays, n, hits, miss, counter, lanes)));
   return 0;
 }
 
