@@ -492,29 +492,46 @@ __global__ void __launch_bounds__(BLK) k_seg_leaves_aabbs(const float* __restric
   seg_reduce_box(b, valid, s, s_block, total_keys, status);
 }
 
+// Every scene's scale, once: three double-precision divisions and the float
+// pieces of the grid, which cost a block more than its 256 codes.
+__global__ void __launch_bounds__(BLK) k_seg_scales(const int* total_keys, uint32_t n_seg, int wide,
+                                                    Scale* __restrict__ scales) {
+  grid_dep_wait();
+  const uint32_t s = blockIdx.x * BLK + threadIdx.x;
+  if (s < n_seg) scales[s] = make_scale(total_keys + 8 * (size_t)s, wide ? GRID128 : GRID64);
+}
+
+// Codes of every scene's leaves, grid-stride over blocks of BLK leaves (one
+// wave).  Most blocks of leaves lie in one scene, whose scale the block keeps in
+// shared memory; the others' leaves read their own from the table.  With the
+// scale computed by each block: 145 us for 3.5M leaves of 96 scenes, now 56 (the
+// batch 5936 -> 5844 us).
 template <bool WIDE>
 __global__ void __launch_bounds__(BLK) k_seg_morton(const Bvh2Node* __restrict__ leaves,
                                                     const uint32_t* __restrict__ prim_start, uint32_t n_seg, uint32_t n,
-                                                    const int* total_keys, void* __restrict__ codes) {
+                                                    const Scale* __restrict__ scales, void* __restrict__ codes) {
   grid_dep_wait();
-  // the scale of the block's first scene once per block (most blocks lie in
-  // one scene); leaves of other scenes compute their own
   __shared__ Scale s_scale;
-  __shared__ uint32_t s_first;
-  const uint32_t i = blockIdx.x * BLK + threadIdx.x;
-  if (threadIdx.x == 0) {
-    s_first = seg_find(prim_start, n_seg, min(blockIdx.x * BLK, n - 1));
-    s_scale = make_scale(total_keys + 8 * (size_t)s_first, WIDE ? GRID128 : GRID64);
+  static_assert(sizeof(Scale) % 4 == 0 && sizeof(Scale) / 4 <= BLK, "a word of the scale per thread");
+  uint32_t held = OBVHS_INVALID, held_end = 0;  // (block-uniform) the scene in s_scale
+  for (uint32_t i0 = blockIdx.x * BLK; i0 < n; i0 += gridDim.x * BLK) {
+    if (held == OBVHS_INVALID || i0 >= held_end) {
+      held = seg_find(prim_start, n_seg, i0);
+      held_end = __ldg(&prim_start[held + 1]);
+      __syncthreads();  // the previous scene's readers are done
+      if (threadIdx.x < sizeof(Scale) / 4)
+        reinterpret_cast<uint32_t*>(&s_scale)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&scales[held])[threadIdx.x];
+      __syncthreads();
+    }
+    const uint32_t i = i0 + threadIdx.x;
+    if (i >= n) continue;
+    const Scale& sc = i < held_end ? s_scale : scales[seg_find(prim_start, n_seg, i)];
+    const Bvh2Node nd = ld_node(&leaves[i]);
+    if (WIDE)
+      static_cast<U128*>(codes)[i] = morton128_of(nd, sc);
+    else
+      static_cast<unsigned long long*>(codes)[i] = morton64_of(nd, sc);
   }
-  __syncthreads();
-  if (i >= n) return;
-  const uint32_t s = seg_find(prim_start, n_seg, i);
-  const Scale sc = s == s_first ? s_scale : make_scale(total_keys + 8 * (size_t)s, WIDE ? GRID128 : GRID64);
-  const Bvh2Node nd = ld_node(&leaves[i]);
-  if (WIDE)
-    static_cast<U128*>(codes)[i] = morton128_of(nd, sc);
-  else
-    static_cast<unsigned long long*>(codes)[i] = morton64_of(nd, sc);
 }
 
 // Scene of each sorted leaf (its value is the leaf's global position), for
@@ -2260,10 +2277,14 @@ int ploc_seg_device(BuildCtx& c, const SegLayout& L, const Bvh2Node* leaves, con
   void* codes = s.get(SLOT_KEYS, (size_t)n * (precision ? sizeof(U128) : sizeof(unsigned long long)));
   if (!codes) return c.fail(OBVHS_ERR_OOM, "scratch");
   const uint32_t g = div_up<uint32_t>(n, BLK);
+  Scale* scales = (Scale*)s.get(SLOT_ARRIVE, (size_t)S * sizeof(Scale));  // (reinsertion's, free until then)
+  if (!scales) return c.fail(OBVHS_ERR_OOM, "scratch");
+  KLAUNCH("k_seg_scales", launch_k(k_seg_scales, div_up<uint32_t>(S, BLK), BLK, 0, c.stream, total_keys, S, precision, scales));
+  const uint32_t gm = std::min<uint32_t>(g, (uint32_t)std::max(c.num_sms, 1) * 8u);
   if (precision)
-    KLAUNCH("k_seg_morton", launch_k(k_seg_morton<true>, g, BLK, 0, c.stream, leaves, L.d_prim_start, S, n, total_keys, codes));
+    KLAUNCH("k_seg_morton", launch_k(k_seg_morton<true>, gm, BLK, 0, c.stream, leaves, L.d_prim_start, S, n, scales, codes));
   else
-    KLAUNCH("k_seg_morton", launch_k(k_seg_morton<false>, g, BLK, 0, c.stream, leaves, L.d_prim_start, S, n, total_keys, codes));
+    KLAUNCH("k_seg_morton", launch_k(k_seg_morton<false>, gm, BLK, 0, c.stream, leaves, L.d_prim_start, S, n, scales, codes));
   CK(cudaGetLastError());
   // Morton order over all leaves, then a stable pass on the scene index: each
   // scene's leaves in its own Morton order (ties by position), scenes in turn
