@@ -392,12 +392,15 @@ int seg_pipeline(BuildCtx& c, const float* const* tris, const uint32_t* n_tris, 
   if (*c.h_status) return take_status(c);
   BuildReadback* rb = reinterpret_cast<BuildReadback*>(static_cast<char*>(c.h_small) + READBACK_OFFSET);
   std::memset(rb, 0, sizeof(BuildReadback));
-  r = reinsertion_seg_device(c, nodes, L, h_passes.data(), p->reinsertion_batch_ratio, upload, &rb->applied);
+  bool parents_ready = false;
+  r = reinsertion_seg_device(c, nodes, L, h_passes.data(), p->reinsertion_batch_ratio, upload, &rb->applied,
+                             &parents_ready);
   if (r) return upload_err ? c.cuda_fail(upload_err, "table upload") : r;
   stages.mark(c.stream);
   const uint32_t mp = p->max_prims_per_leaf < 1 ? 1 : (p->max_prims_per_leaf > 3 ? 3 : p->max_prims_per_leaf);
   uint32_t expected = 0;
-  r = cwbvh_seg_device(c, nodes, pidx, L, mp, 1, tris, n_tris, split ? 1 : 0, upload, outs, &rb->emitted, &expected);
+  r = cwbvh_seg_device(c, nodes, pidx, L, mp, 1, tris, n_tris, split ? 1 : 0, upload, outs, &rb->emitted, &expected,
+                       parents_ready);
   auto drop = [&]() {
     for (auto* o : outs) obvhs_cwbvh_free(o);
     outs.clear();

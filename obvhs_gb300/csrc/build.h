@@ -385,9 +385,10 @@ int seg_root_parents_device(BuildCtx& c, const SegLayout& L, uint32_t* parents);
 // The 16 reinsertion passes of every scene (reinsertion.rs:101-115 per
 // scene), each pass one candidate sort, one search and one resolve launch for
 // all scenes.  h_passes: each scene's PLOC passes (its stack bound).  The
-// applied total is copied to pinned *applied_deferred.
+// applied total is copied to pinned *applied_deferred.  *parents_ready: whether
+// SLOT_PARENTS holds the resulting trees' parent links.
 int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, const uint32_t* h_passes, float ratio,
-                           SegTableUpload upload, uint32_t* applied_deferred);
+                           SegTableUpload upload, uint32_t* applied_deferred, bool* parents_ready);
 
 // cwbvh.cu
 // With `emitted_deferred` (pinned) the number of emitted nodes is copied there
@@ -411,7 +412,7 @@ int cwbvh_order_children_device(BuildCtx& c, obvhs_cwbvh* b, const float* prims6
 int cwbvh_seg_device(BuildCtx& c, const Bvh2Node* nodes, const uint32_t* pidx_in, const SegLayout& L,
                      uint32_t max_prims, int order_children, const float* const* h_tris, const uint32_t* h_ntris,
                      int uses_spatial_splits, SegTableUpload upload, std::vector<obvhs_cwbvh*>& outs,
-                     uint32_t* emitted_deferred, uint32_t* emitted_expected);
+                     uint32_t* emitted_deferred, uint32_t* emitted_expected, bool parents_ready);
 
 // traverse.cu
 // One scene's triangles to reorder: tris[pidx[k]] -> out[k], k < its primitive count.

@@ -1711,8 +1711,9 @@ int seg_root_parents_device(BuildCtx& c, const SegLayout& L, uint32_t* parents) 
 }
 
 int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, const uint32_t* h_passes, float ratio,
-                           SegTableUpload upload, uint32_t* applied_deferred) {
+                           SegTableUpload upload, uint32_t* applied_deferred, bool* parents_ready) {
   *applied_deferred = 0;
+  *parents_ready = false;
   const uint32_t S = L.n_seg, len = L.n_slots;
   if (len == 0 || !(ratio > 0.0f)) return 0;
   constexpr uint32_t NSEQ = 16;
@@ -1782,6 +1783,7 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
   if (r) return r;
   r = seg_root_parents_device(c, L, B.parents);
   if (r) return r;
+  *parents_ready = true;  // (kept up to date by every pass)
   const StackModes modes{all_clamp ? nullptr : d_mode, L.d_node_start, S};
   const int digits = 4 + (S <= 256 ? 1 : 2);
   for (uint32_t ri = 0; ri < NSEQ; ri++) {
