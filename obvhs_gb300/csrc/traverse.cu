@@ -1208,10 +1208,9 @@ __device__ __forceinline__ void write_bvh_tri(const float* tris, uint32_t n_tris
   const float3 e1 = make_float3(v0.x - v1.x, v0.y - v1.y, v0.z - v1.z);
   const float3 e2 = make_float3(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z);
   const float3 n = make_float3(e1.y * e2.z - e1.z * e2.y, e1.z * e2.x - e1.x * e2.z, e1.x * e2.y - e1.y * e2.x);
-  out[4 * (size_t)k] = make_float4(v0.x, v0.y, v0.z, __uint_as_float(pidx[k]));
-  out[4 * (size_t)k + 1] = make_float4(e1.x, e1.y, e1.z, n.x);
-  out[4 * (size_t)k + 2] = make_float4(e2.x, e2.y, e2.z, n.y);
-  out[4 * (size_t)k + 3] = make_float4(n.z, 0.0f, 0.0f, 0.0f);
+  st_256(&out[4 * (size_t)k], make_float4(v0.x, v0.y, v0.z, __uint_as_float(pidx[k])),
+         make_float4(e1.x, e1.y, e1.z, n.x));
+  st_256(&out[4 * (size_t)k + 2], make_float4(e2.x, e2.y, e2.z, n.y), make_float4(n.z, 0.0f, 0.0f, 0.0f));
 }
 
 __global__ void k_reorder_tris(const float* __restrict__ tris, uint32_t n_tris, const uint32_t* __restrict__ pidx,
