@@ -525,8 +525,15 @@ struct CwRay {
 // per thread, entry k of thread t at [k][t]: consecutive threads' entries
 // are adjacent, so a warp's pushes and pops are conflict-free) instead of
 // the thread's local memory.  Same loop, same results.
+// Closest hits on compressed triangles ask for 66 registers, one step above
+// the 64 that let an SM hold 1,024 threads; held to 64 it spills nothing and
+// 8M rays on 8M triangles take 7654 -> 7182 us, 2M on 2M 1545 -> 1484, 1.5M on
+// 300k 1136 -> 1095 (camera rays on 1M 1681 -> 1672, on 500k 683 -> 687, the
+// runs 679-688).  The multi-BVH form (69) spills 22 bytes at 64 and gains
+// nothing (96 scenes 5716 -> 5709 us, 20 scenes 1879 -> 1886), so it and the
+// others are left to the compiler (0: no bound).
 template <int MODE, bool CTRI = false, bool MULTI = false, int TB = TBLK, bool SST = false, bool FEW = false>
-__global__ void __launch_bounds__(TB) k_traverse(const CwNode* __restrict__ nodes_in, uint32_t n_nodes_in,
+__global__ void __launch_bounds__(TB, MODE == 0 && CTRI && !FEW ? 1024 / TB : 0) k_traverse(const CwNode* __restrict__ nodes_in, uint32_t n_nodes_in,
                                                    const float4* __restrict__ tris_in, uint32_t n_prims_in,
                                                    const float4* __restrict__ rays,
                                                    uint32_t nrays, uint2* __restrict__ hits, uint8_t* __restrict__ miss,
