@@ -142,9 +142,10 @@ __global__ void __launch_bounds__(BLK) k_cand_keys(const Bvh2Node* __restrict__ 
 // one launch computes every scene's keys, sorts them stably and writes each
 // scene's first candidates, in place of a global sort of all scenes' 64-bit
 // (scene, key) words (clear, histogram, five digit passes, gather).  Bound by
-// the block's barriers and the match / shared-memory chain of a digit pass (16
-// us for one scene of 1,000-7,000 candidates); a batch runs as many blocks as
-// scenes.  96 scenes of 1k-200k triangles 7432 -> 7010 us.  (For one tree a
+// the block's barriers and the ballot / shared-memory chain of a digit pass (in a
+// batch of 96 scenes 31.8 us a launch, 39.1 with match.any in place of the
+// ballots); a batch runs as many blocks as scenes.  96 scenes of 1k-200k
+// triangles 7432 -> 7010 us, then 5612 -> 5573 with the ballots.  (For one tree a
 // block takes longer than the global sort above 8,000 candidates: 100k
 // triangles, slow build, 2789 -> 2894 us.)  A thread keeps up to CS_ITEMS
 // candidates in registers; warp w owns the contiguous candidates [w * 32 * I,
@@ -225,7 +226,12 @@ __device__ __forceinline__ void sort_candidates(const Bvh2Node* nodes, uint32_t 
       if ((uint32_t)r >= items) break;
       const bool valid = base_i + 32u * r < n;
       const uint32_t d = valid ? (key[r] >> shift) & 0xffu : 256u;
-      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+      for (int b = 0; b < 8; b++) {  // as in the radix passes: cheaper than match.any
+        const uint32_t bit = (uint32_t)((int32_t)(d << (31 - b)) >> 31);
+        peers &= ~(__ballot_sync(0xffffffffu, bit != 0u) ^ bit);
+      }
       const uint32_t lrank = __popc(peers & lt_mask);
       const uint32_t before = valid ? wh[d] : 0u;
       __syncwarp();
