@@ -620,6 +620,10 @@ __global__ void __launch_bounds__(BLK) k_costs_oct(const Bvh2Node* __restrict__ 
     uint32_t first = 0;
     if (climbing && sub == 0) first = atom_add_acq_rel(&flags[p], 1u) == 0 ? 1u : 0u;
     first = __shfl_sync(FULL_MASK, first, 0, 8);
+    // the arrival acquires the sibling's record for its own lane alone and a
+    // shuffle orders no memory: the barrier passes it on to the octet's others,
+    // as the one above hands their stores to the arrival
+    __syncwarp();
     if (first) climbing = false;  // the sibling's climb continues
     const uint32_t f = node_first(pn);
     const bool own_left = c == f;
