@@ -1143,6 +1143,9 @@ __global__ void __launch_bounds__(EMIT_TB, 7) k_emit_all(EmitArgs a) {
     waits = 0;
     ns = 32;
     OctNode s;
+    // the octet's first lane has seen the flag: its other lanes' reads come after
+    // that through this barrier (a shuffle orders no memory)
+    __syncwarp();
     if (go) {
       __threadfence();
       // through L2: this SM may hold a stale L1 line of the items array
@@ -1444,6 +1447,7 @@ __global__ void __launch_bounds__(EMIT_THREADS) k_order_children(OrderArgs a) {
       __threadfence();
     }
     ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();  // lane 0's fence stands before every lane's reads
     if (!ok) break;
     const uint32_t ni = __ldcg(&a.items[k]);
     if (ni >= a.n_nodes) {

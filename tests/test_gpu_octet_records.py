@@ -37,3 +37,27 @@ def test_repeated_conversions_agree(n, reinserted):
         for k in kept:
             k.free()
         b.free()
+
+
+@pytest.mark.parametrize("n", [300, 20_000])
+def test_repeated_emission_and_child_order_agree(n):
+    """The two work queues, whose items one lane waits for and others read."""
+    import obvhs_gb300 as G
+
+    rng = np.random.default_rng(n + 1)
+    c = rng.uniform(-5, 5, size=(n, 3)).astype(np.float32)
+    h = np.exp(rng.uniform(-6, 0, size=(n, 3))).astype(np.float32)
+    boxes = np.concatenate([c - h, c + h], 1)
+    nodes, order, md, _ = O.ploc(boxes, None, 6, 0, 1)
+    plain, plain_order = O.bvh2_to_cwbvh(nodes, order, 3, False)
+    want = O.cwbvh_order_children(plain, plain_order, boxes)
+    want = want[0] if isinstance(want, tuple) else want
+    with G.Context() as ctx:
+        b = G.Bvh2.upload(nodes, order, md, ctx=ctx)
+        for _ in range(20):
+            cw = G.bvh2_to_cwbvh(b, 3, False)
+            assert cw.download()[0].tobytes() == plain.tobytes()
+            cw.order_children(boxes)
+            assert cw.download()[0].tobytes() == want.tobytes()
+            cw.free()
+        b.free()
