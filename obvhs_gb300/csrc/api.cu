@@ -186,7 +186,7 @@ int build_pipeline(BuildCtx& c, const float* tris, const float* aabbs, uint32_t 
   cw->uses_spatial_splits = split;
   // with no reinsertion the tree is PLOC's own: its pass ranges order the cost pass
   const bool plain_ploc = !(p->reinsertion_batch_ratio > 0.0f) && passes > 0;
-  r = cwbvh_convert_device(c, &b2, mp, 1, cw, &rb->emitted, false, plain_ploc ? passes : 0u);
+  r = cwbvh_convert_device(c, &b2, mp, 1, cw, &rb->emitted, false, plain_ploc ? passes : 0u, true);
   if (r) {
     obvhs_cwbvh_free(cw);
     return r;

@@ -370,13 +370,16 @@ int reinsertion_device(BuildCtx& c, obvhs_bvh2* b, float batch_size_ratio, const
                        uint64_t* applied_out, int64_t root_prims = -1, uint32_t* applied_deferred = nullptr);
 // Parent links of every node (roots: their own).  With `unordered`, also
 // sets *unordered (zeroed by the caller) when some inner node's children are
-// not both at higher indices than the node.
+// not both at higher indices than the node.  With `odd` (zeroed by the caller,
+// `parents` filled with OBVHS_INVALID by it) the nodes may be any: nodes that
+// none names keep OBVHS_INVALID, and *odd is set where the links are not a
+// tree's.
 // The traversal launch form for (threads per block, group stack in shared
 // memory); -1 when there is none.
 int traversal_form_index(uint32_t block, int smem_stack);
 
 int compute_parents_device(BuildCtx& c, const Bvh2Node* nodes, uint32_t n_nodes, uint32_t* parents,
-                           uint32_t* unordered = nullptr);
+                           uint32_t* unordered = nullptr, uint32_t* odd = nullptr);
 // Copies a host table to the device (stream-ordered, from pinned staging);
 // returns the device address or null.
 typedef std::function<uint32_t*(const void* src, size_t bytes)> SegTableUpload;
@@ -395,9 +398,12 @@ int reinsertion_seg_device(BuildCtx& c, Bvh2Node* nodes, const SegLayout& L, con
 // asynchronously; the caller compares it with out->n_nodes after its final
 // synchronisation and checks the status word.
 // ploc_passes > 0: the tree is exactly as this context's last PLOC build
-// left it after that many passes (its pass ranges are valid).
+// left it after that many passes (its pass ranges are valid).  sound: this
+// context has just built the tree without an error, so its links are a tree's;
+// else they are checked first.
 int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, int order_children, obvhs_cwbvh* out,
-                         uint32_t* emitted_deferred = nullptr, bool exact_aabbs = false, uint32_t ploc_passes = 0);
+                         uint32_t* emitted_deferred = nullptr, bool exact_aabbs = false, uint32_t ploc_passes = 0,
+                         bool sound = false);
 // CwBvh::order_children (node < 0) or order_node_children(node) on the
 // device; prims6: the primitives' boxes (n_prims x 6 floats, device), in
 // original order or, with direct_layout, in primitive_indices order.

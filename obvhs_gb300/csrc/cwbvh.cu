@@ -244,6 +244,7 @@ struct CostClimb {
       __stcg(&erec[i], make_uint4(0u, 0u, 1u, 0u));
       return false;
     }
+    if (p >= n) return false;  // (OBVHS_INVALID) a leaf that no node names: in no tree
     own = leaf_rec(nd);
     own_leaf = true;
     c = i;
@@ -285,7 +286,7 @@ struct CostClimb {
     own_list = list;
     own_leaf = false;
     __stcg(&erec[p], make_uint4(own.meta, aggn0, own.nprim, 0u));
-    if (up == p) return true;
+    if (up == p || up >= n) return true;  // a root, or the top of nodes that no tree names
     c = p;
     p = up;
     return false;
@@ -355,7 +356,20 @@ __device__ void costs_ordered(const Bvh2Node* __restrict__ nodes, const uint32_t
       continue;
     }
     const uint32_t f = node_first(nd);
-    if (f + 1 >= n_all || f < i) {  // an inert pad (children out of range): nothing to compute
+    if (f >= n_all - 1 || f < i) {
+      // an inert pad (children out of range).  A node above one, in a tree made
+      // elsewhere, has no finite distribution and too many primitives for a leaf
+      CostRec none;
+#pragma unroll
+      for (int k = 0; k < 7; k++) {
+        none.cost[k] = __int_as_float(0x7f800000);
+        none.contrib[k] = AGG_INVALID;
+      }
+      none.meta = 0;
+      none.nprim = 4;
+      st_rec(&crec[i], none);
+      __stcg(&erec[i], make_uint4(0u, AGG_INVALID, 4u, 0u));
+      __threadfence();
       atomicExch(&flags[i], 1u);
       continue;
     }
@@ -465,12 +479,14 @@ constexpr uint32_t COST_REFILL_IDLE = 8;
 // ends counts itself idle, and once COST_REFILL_IDLE lanes of its warp are
 // idle they take new nodes while the others keep climbing.  Climbs of very
 // different lengths so never hold a block (or a warp) for their longest
-// member.  `next` starts at 0.
+// member.  `next` starts at 0.  A launch that finds 0 at `only_if` does nothing.
 __global__ void __launch_bounds__(BLK) k_costs(const Bvh2Node* __restrict__ nodes, const uint32_t* __restrict__ parents,
                                                const uint32_t* __restrict__ pidx_in, uint32_t n, uint32_t max_prims,
                                                CostRec* crec, EmitRec* erec, uint4* small, uint32_t* flags,
-                                               uint32_t* next, const uint32_t* unordered, uint32_t* status) {
+                                               uint32_t* next, const uint32_t* unordered, uint32_t* status,
+                                               const uint32_t* only_if) {
   grid_dep_wait();
+  if (only_if && *only_if == 0) return;
   if (unordered && *unordered == 0) {  // (null: not known to be ordered)
     costs_ordered(nodes, parents, pidx_in, n, max_prims, crec, erec, small, flags, next, status, n);
     return;
@@ -551,12 +567,15 @@ __device__ __forceinline__ uint32_t oct_bits(uint32_t ballot, int lane) { return
 // instead of 330 dependent ones in one thread, and a record is two coalesced
 // 32-byte accesses.  Same records, same arithmetic per slot, as inner_rec.
 // 4k nodes after reinsertion 95 -> 33 us, 20k nodes from PLOC (ready flags
-// polled level by level before) 120 -> 41 us.
+// polled level by level before) 120 -> 41 us.  The climb follows parent links, so
+// a launch that finds *odd set (links that are not a tree's) leaves the tree to
+// k_costs, which takes shared and unnamed nodes where they are in node order.
 __global__ void __launch_bounds__(BLK) k_costs_oct(const Bvh2Node* __restrict__ nodes, const uint32_t* __restrict__ parents,
                                                    const uint32_t* __restrict__ pidx_in, uint32_t n, uint32_t max_prims,
                                                    CostRec* crec, EmitRec* erec, uint4* small, uint32_t* flags,
-                                                   uint32_t* status) {
+                                                   uint32_t* status, const uint32_t* odd) {
   grid_dep_wait();
+  if (odd && *odd) return;
   const float INF = __int_as_float(0x7f800000);
   const int lane = threadIdx.x & 31, sub = lane & 7;
   const uint32_t n_oct = gridDim.x * (BLK / 8);
@@ -582,7 +601,7 @@ __global__ void __launch_bounds__(BLK) k_costs_oct(const Bvh2Node* __restrict__ 
         __stcg(&small[i], list);
         if (p == i) __stcg(&erec[i], make_uint4(0u, 0u, 1u, 0u));  // a leaf root: one CWBVH node
       }
-      if (p == i) continue;
+      if (p == i || p >= n) continue;  // a leaf root, or (OBVHS_INVALID) a leaf that no node names
       const CostRec r = leaf_rec(nd);
       cost = r.cost[0];
       contrib = 0;
@@ -714,7 +733,7 @@ __global__ void __launch_bounds__(BLK) k_costs_oct(const Bvh2Node* __restrict__ 
       meta = m;
       nprim = np;
       leaf = false;
-      climbing = up != p;
+      climbing = up != p && up < n;
       c = p;
       p = up;
     }
@@ -1540,14 +1559,17 @@ static const uint32_t* ceil_log2_thresholds() {
 }
 
 int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, int order_children, obvhs_cwbvh* out,
-                         uint32_t* emitted_deferred, bool exact_aabbs, uint32_t ploc_passes) {
+                         uint32_t* emitted_deferred, bool exact_aabbs, uint32_t ploc_passes, bool sound) {
   out->n_nodes = 0;
   out->n_prims = 0;
   const uint32_t n = b->n_nodes;
   if (n == 0) return 0;
   Scratch& s = c.scratch;
   uint32_t* parents = (uint32_t*)s.get(SLOT_PARENTS, (size_t)n * 4);
-  uint32_t* flags = (uint32_t*)s.get(SLOT_FLAGS, (size_t)n * 4 + 8);  // + k_costs' node counter, order flag
+  // + k_costs' node counter, order flag; whether the links are not a tree's
+  const size_t flag_bytes = (size_t)n * 4 + 12;
+  uint32_t* flags = (uint32_t*)s.get(SLOT_FLAGS, flag_bytes);
+  uint32_t* odd = flags + n + 2;
   CostRec* crec = (CostRec*)s.get(SLOT_DECISIONS, (size_t)n * sizeof(CostRec));
   EmitRec* erec = (EmitRec*)s.get(SLOT_CW_META, (size_t)n * sizeof(EmitRec));
   uint4* small = (uint4*)s.get(SLOT_CW_SMALL, (size_t)n * sizeof(uint4));
@@ -1556,12 +1578,23 @@ int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, i
   // the tree came straight from this context's last PLOC build: cost it
   // range by range (a cooperative launch), unless the GPU is shared
   const bool ranges = ploc_passes > 0 && ploc_passes < PLOC_PASS_REC && c.ploc_pass_ins && !gpu_shared(c);
+  // a tree from elsewhere: links that nothing writes lead nowhere, and a root
+  // whose record is never computed has no distribution
+  if (!sound) {
+    CK(cudaMemsetAsync(parents, 0xff, (size_t)n * 4, c.stream));
+    CK(cudaMemsetAsync(erec, 0xff, sizeof(EmitRec), c.stream));
+  }
   if (n <= COST_OCT_MAX) {
-    CK(cudaMemsetAsync(flags, 0, (size_t)n * 4 + 8, c.stream));
-    int r = compute_parents_device(c, b->nodes, n, parents);
+    CK(cudaMemsetAsync(flags, 0, flag_bytes, c.stream));
+    int r = sound ? compute_parents_device(c, b->nodes, n, parents)
+                  : compute_parents_device(c, b->nodes, n, parents, flags + n + 1, odd);
     if (r) return r;
     KLAUNCH("k_costs_oct", launch_k(k_costs_oct, cost_oct_grid(c, n), BLK, 0, c.stream, b->nodes, parents, b->prim_indices,
-                                    n, max_prims, crec, erec, small, flags, c.d_status));
+                                    n, max_prims, crec, erec, small, flags, c.d_status,
+                                    sound ? (const uint32_t*)nullptr : odd));
+    if (!sound)
+      KLAUNCH("k_costs", launch_k(k_costs, cost_grid(c, n), BLK, 0, c.stream, b->nodes, parents, b->prim_indices, n,
+                                  max_prims, crec, erec, small, flags, flags + n, flags + n + 1, c.d_status, odd));
   } else if (ranges) {  // (the kernel clears the flags it uses)
     CostRangeArgs ra{b->nodes, b->prim_indices, c.ploc_pass_ins, n, max_prims, ploc_passes, crec, erec, small,
                      c.d_status};
@@ -1570,11 +1603,12 @@ int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, i
     void* args[] = {&ra, &fl, &nx};
     KLAUNCH("k_costs", CK(coop_launch(c, (const void*)k_costs_ranges, cost_range_grid(c), BLK, args, 0)));
   } else {
-    CK(cudaMemsetAsync(flags, 0, (size_t)n * 4 + 8, c.stream));
+    CK(cudaMemsetAsync(flags, 0, flag_bytes, c.stream));
     int r = compute_parents_device(c, b->nodes, n, parents, flags + n + 1);
     if (r) return r;
     KLAUNCH("k_costs", launch_k(k_costs, cost_grid(c, n), BLK, 0, c.stream, b->nodes, parents, b->prim_indices, n,
-                                max_prims, crec, erec, small, flags, flags + n, flags + n + 1, c.d_status));
+                                max_prims, crec, erec, small, flags, flags + n, flags + n + 1, c.d_status,
+                                (const uint32_t*)nullptr));
   }
   CK(cudaGetLastError());
   // sizes of the whole tree: the root's aggregate (a leaf root is one node)
@@ -1585,7 +1619,9 @@ int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, i
   if (*c.h_status)
     return c.fail(OBVHS_ERR_BAD_INPUT, "BVH2 cannot be converted (a leaf holds more than one primitive)");
   const bool root_leaf = n == 1;
-  if (!root_leaf && root.y == AGG_INVALID)
+  if (root.z == OBVHS_INVALID)
+    return c.fail(OBVHS_ERR_BAD_INPUT, "BVH2 cannot be converted (its links are not a tree's)");
+  if (root.y == AGG_INVALID)
     return c.fail(OBVHS_ERR_BAD_INPUT, "BVH2 cannot be converted (no finite distribution of the root)");
   const uint32_t n_cw = root_leaf ? 1 : 1 + root.y;
   const uint32_t n_pr = root.z;
@@ -1706,7 +1742,7 @@ int cwbvh_seg_device(BuildCtx& c, const Bvh2Node* nodes, const uint32_t* pidx_in
   }
   KLAUNCH("k_costs", launch_k(k_costs, cost_grid(c, n), BLK, 0, c.stream, nodes, parents, pidx_in, n, max_prims, crec,
                               erec, small, flags, flags + n, parents_ready ? (const uint32_t*)nullptr : flags + n + 1,
-                              c.d_status));
+                              c.d_status, (const uint32_t*)nullptr));
   KLAUNCH("k_seg_roots_out", launch_k(k_seg_roots_out, div_up<uint32_t>(S, BLK), BLK, 0, c.stream,
                                  nodes, erec, L.d_prim_start, L.d_node_start, S, roots));
   CK(cudaGetLastError());

@@ -49,21 +49,31 @@ struct Reins {
 // inner node's children do not both lie above it in the array (trees straight
 // from PLOC always have them above: pairs are written top down, a parent
 // after its children).  Nodes whose children are out of range (the inert pads
-// of segmented builds) link nothing.
+// of segmented builds) link nothing.  With `odd` non-null the array may hold
+// anything (a tree made elsewhere) and `parents` starts as OBVHS_INVALID: *odd
+// is set when a node is named twice, the root is named, or a child is out of
+// range.  Where it stays 0, the part that the root reaches is a tree whose links
+// agree, and any other node's links end at OBVHS_INVALID or in a ring that no
+// climb enters.
 __global__ void k_parents(const Bvh2Node* __restrict__ nodes, uint32_t n, uint32_t* __restrict__ parents,
-                          uint32_t* unordered) {
+                          uint32_t* unordered, uint32_t* odd) {
   grid_dep_wait();
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (i == 0) parents[0] = 0;
   Bvh2Node nd = ld_node(&nodes[i]);
   if (node_prims(nd) == 0) {
-    uint32_t f = node_first(nd);
-    if (f + 1 < n) {
+    const uint32_t f = node_first(nd);
+    const bool in_range = f < n - 1;  // (f + 1 would wrap)
+    if (in_range && odd) {
+      const uint32_t a = atomicExch(&parents[f], i), b = atomicExch(&parents[f + 1], i);
+      if (a != OBVHS_INVALID || b != OBVHS_INVALID) *odd = 1u;
+    } else if (in_range) {
       parents[f] = i;
       parents[f + 1] = i;
     }
-    if (unordered && f <= i && f + 1 < n) *unordered = 1u;
+    if (odd && (!in_range || f == 0)) *odd = 1u;
+    if (unordered && in_range && f <= i) *unordered = 1u;
   }
 }
 
@@ -1610,10 +1620,10 @@ int reinsertion_setup_kernels() {
 }
 
 int compute_parents_device(BuildCtx& c, const Bvh2Node* nodes, uint32_t n_nodes, uint32_t* parents,
-                           uint32_t* unordered) {
+                           uint32_t* unordered, uint32_t* odd) {
   if (!n_nodes) return 0;
   KLAUNCH("k_parents", launch_k(k_parents, div_up<uint32_t>(n_nodes, BLK), BLK, 0, c.stream, nodes, n_nodes, parents,
-                                unordered));
+                                unordered, odd));
   CK(cudaGetLastError());
   return 0;
 }
