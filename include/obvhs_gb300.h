@@ -365,7 +365,8 @@ OBVHS_API int obvhs_ray_traverse_batches(obvhs_ctx* ctx, const obvhs_cwbvh* cons
  * `block` threads per block (64, 128 or 256) and keep each ray's 32-entry
  * group stack in local memory, or in shared memory (smem_stack = 1, blocks
  * of 64 or 128).  Results are identical in every form; (0, 0) restores the
- * default (128, local).  Other values return OBVHS_ERR_INVALID_ARG. */
+ * default (128, local), in which a call of few rays gives each warp fewer than
+ * 32 of them.  Other values return OBVHS_ERR_INVALID_ARG. */
 OBVHS_API int obvhs_ctx_set_traversal_config(obvhs_ctx* ctx, uint32_t block, int smem_stack);
 
 /* ---- device wait limits -------------------------------------------------- */

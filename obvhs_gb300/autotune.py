@@ -73,6 +73,8 @@ def tune_segmented(scenes, rays, ray_owner, base: BvhBuildParams, ctx=None, radi
 def tune_traversal(trace, ctx, reps: int = 3, forms=None):
     """Times `trace()` (one traversal call on `ctx`, device work synchronised
     after it) in every traversal launch form; leaves ctx in the default form.
+    The call should have as many rays as the calls the choice is for: the
+    default form alone spreads a call of few rays over more warps.
     Returns {"block", "smem_stack", "ms": {"<block><L|S>": best ms}}."""
     from . import bvh
 

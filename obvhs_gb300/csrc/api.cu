@@ -669,7 +669,7 @@ int obvhs_ctx_set_shared_gpu(obvhs_ctx* c, int shared) {
 
 int obvhs_ctx_set_traversal_config(obvhs_ctx* c, uint32_t block, int smem_stack) {
   if (!c) return OBVHS_ERR_INVALID_ARG;
-  const int f = traversal_form_index(block, smem_stack);
+  const int f = trav_form_index(block, smem_stack);
   if (f < 0) return c->fail(OBVHS_ERR_INVALID_ARG, "traversal config: block 64/128/256 with a local stack, or 64/128 "
                                                    "with a shared-memory stack (0, 0: the default)");
   c->trav_form = f;

@@ -14,6 +14,7 @@
 
 #include "../../include/obvhs_gb300.h"
 #include "common.cuh"
+#include "traverse_form.h"
 
 // Clusters left when PLOC switches to the single-CTA shared-memory tail.
 constexpr uint32_t TAIL_MAX = 2048;
@@ -374,10 +375,6 @@ int reinsertion_device(BuildCtx& c, obvhs_bvh2* b, float batch_size_ratio, const
 // `parents` filled with OBVHS_INVALID by it) the nodes may be any: nodes that
 // none names keep OBVHS_INVALID, and *odd is set where the links are not a
 // tree's.
-// The traversal launch form for (threads per block, group stack in shared
-// memory); -1 when there is none.
-int traversal_form_index(uint32_t block, int smem_stack);
-
 int compute_parents_device(BuildCtx& c, const Bvh2Node* nodes, uint32_t n_nodes, uint32_t* parents,
                            uint32_t* unordered = nullptr, uint32_t* odd = nullptr);
 // Copies a host table to the device (stream-ordered, from pinned staging);

@@ -564,29 +564,6 @@ __global__ void __launch_bounds__(TB, MODE == 0 && CTRI && !FEW ? 1024 / TB : 0)
   voted_rays<decltype(ray), TB>(ray, nrays, next_ray, yield, FEW ? lanes : 32u);
 }
 
-// The traversal launch forms a context can choose (obvhs_ctx_set_traversal_config):
-// block size and stack placement.  Form 0 is the default.
-struct TravForm {
-  int block;
-  bool smem_stack;
-};
-constexpr TravForm TRAV_FORMS[] = {{128, false}, {64, false}, {256, false}, {64, true}, {128, true}};
-constexpr int N_TRAV_FORMS = 5;
-
-// Rays a warp takes at a time.  A call of few rays is a chain of dependent
-// loads per ray, and a warp takes the time of all its rays' different steps
-// together, so they are spread: one ray a warp while that gives each of the
-// SMs' four schedulers at most two warps, then two, four, ... (1,000 host rays
-// on 10k triangles 88.6 -> 78.9 us the call, 3,000 on 100k 111.6 -> 105.2,
-// 14,400 149 -> 144; from 30,000 rays even.  Four warps a scheduler: 30,000
-// rays 159 -> 167 us; one: 3,000 rays 108 us).  The kernels that take 32 are
-// compiled apart: with the count in a register they ran 1-1.6 % slower.
-inline uint32_t rays_per_warp(const BuildCtx& c, uint32_t n) {
-  uint32_t lanes = 1;
-  while (lanes < 32 && (uint64_t)lanes * c.num_sms * 8 < n) lanes *= 2;
-  return lanes;
-}
-
 // Launches k_traverse<MODE, false, MULTI> in form f as a persistent grid
 // (resident blocks, or fewer for a small batch).
 template <int MODE, bool MULTI, int TB, bool SST, bool FEW = false>
@@ -619,7 +596,7 @@ template <int MODE, bool MULTI>
 cudaError_t launch_trav(BuildCtx& c, uint32_t n, const CwNode* nodes, uint32_t n_nodes, const float4* tris,
                         uint32_t n_prims, const float4* rays, uint2* hits, uint8_t* miss, uint32_t* counter,
                         const BlasDesc* dd, const uint32_t* ray_bvh, uint32_t n_bvh) {
-  const uint32_t lanes = rays_per_warp(c, n);
+  const uint32_t lanes = trav_rays_per_warp(n, c.num_sms, c.trav_form);
   if (lanes < 32)
     return launch_trav_form<MODE, MULTI, TBLK, false, true>(c, n, nodes, n_nodes, tris, n_prims, rays, hits, miss, counter,
                                                             dd, ray_bvh, n_bvh, lanes);
@@ -1417,7 +1394,7 @@ int traverse_compressed_device(BuildCtx& c, const obvhs_cwbvh* bvh, const float*
   uint32_t* counter = (uint32_t*)c.scratch.get(SLOT_OUTPUT, 16);
   if (!counter) return c.fail(OBVHS_ERR_OOM, "scratch");
   CK(cudaMemsetAsync(counter, 0, 4, c.stream));
-  const uint32_t lanes = rays_per_warp(c, n);
+  const uint32_t lanes = trav_rays_per_warp(n, c.num_sms, 0);  // (the only form)
   if (lanes < 32)
     CK((mode == 0 ? launch_ctri<0, true>(c, bvh, rays, n, hits, miss, counter, lanes)
                   : launch_ctri<1, true>(c, bvh, rays, n, hits, miss, counter, lanes)));
@@ -1513,12 +1490,4 @@ int query_device(BuildCtx& c, int structure, int kind, const void* nodes, uint32
   }
 #undef QLAUNCH
   return 0;
-}
-
-// Maps (block, smem_stack) to a launch form of the traversal kernels.
-int traversal_form_index(uint32_t block, int smem_stack) {
-  if (block == 0 && !smem_stack) return 0;
-  for (int f = 0; f < N_TRAV_FORMS; f++)
-    if ((uint32_t)TRAV_FORMS[f].block == block && TRAV_FORMS[f].smem_stack == (smem_stack != 0)) return f;
-  return -1;
 }
