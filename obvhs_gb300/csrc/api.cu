@@ -1545,25 +1545,18 @@ static int query_common(obvhs_ctx* cp, int structure, const void* nodes, uint32_
       prim_aabbs ? (const float*)stage_in(c, SLOT_INPUT, prim_aabbs, (size_t)n_prims * 24, device_ptrs, &err) : nullptr;
   if (err) return err;
   uint32_t* doff = offsets;
-  uint32_t* dids = ids;
   if (!device_ptrs) {
     doff = (uint32_t*)c.scratch.get(SLOT_FRONTIER_A, ((size_t)n + 1) * 4);
-    dids = ids ? (uint32_t*)c.scratch.get(SLOT_FRONTIER_B, (size_t)std::max<uint64_t>(capacity, 1) * 4) : nullptr;
-    if (!doff || (ids && !dids)) return c.fail(OBVHS_ERR_OOM, "output staging");
+    if (!doff) return c.fail(OBVHS_ERR_OOM, "output staging");
   }
   float d[3] = {0.0f, 0.0f, 0.0f};
   if (direction) std::memcpy(d, direction, 12);
   const uint32_t oct =
       (d[0] < 0.0f ? 0u : 0x04040404u) | (d[1] < 0.0f ? 0u : 0x02020202u) | (d[2] < 0.0f ? 0u : 0x01010101u);
-  uint32_t total = 0;
-  int r = query_device(c, structure, kind, nodes, n_nodes, pidx, n_pidx, dq, n, dp, n_prims, oct, doff, dids, capacity,
-                       &total);
+  int r = query_device(c, structure, kind, nodes, n_nodes, pidx, n_pidx, dq, n, dp, n_prims, oct, doff, ids,
+                       !device_ptrs, capacity);
   if (r) return r;
-  if (!device_ptrs) {
-    CK(cudaMemcpyAsync(offsets, doff, ((size_t)n + 1) * 4, cudaMemcpyDeviceToHost, c.stream));
-    if (ids && capacity >= total && total)
-      CK(cudaMemcpyAsync(ids, dids, (size_t)total * 4, cudaMemcpyDeviceToHost, c.stream));
-  }
+  if (!device_ptrs) CK(cudaMemcpyAsync(offsets, doff, ((size_t)n + 1) * 4, cudaMemcpyDeviceToHost, c.stream));
   return take_status(c);
 }
 

@@ -1450,8 +1450,7 @@ int traverse_device(BuildCtx& c, const obvhs_cwbvh* bvh, const float* rays, uint
 // capacity >= offsets[n].
 int query_device(BuildCtx& c, int structure, int kind, const void* nodes, uint32_t n_nodes, const uint32_t* pidx,
                  uint32_t n_pidx, const float* queries, uint32_t n, const float* prims, uint32_t n_prims,
-                 uint32_t oct, uint32_t* offsets, uint32_t* ids, uint64_t capacity, uint32_t* total_out) {
-  *total_out = 0;
+                 uint32_t oct, uint32_t* offsets, uint32_t* ids, bool ids_host, uint64_t capacity) {
   CK(cudaMemsetAsync(offsets, 0, 4, c.stream));
   if (n == 0) return 0;
   const uint32_t grid = std::min<uint32_t>(div_up<uint32_t>(n, TBLK), (uint32_t)c.num_sms * 16);
@@ -1483,10 +1482,12 @@ int query_device(BuildCtx& c, int structure, int kind, const void* nodes, uint32
   uint32_t total = 0;
   CK(cudaMemcpyAsync(&total, offsets + n, 4, cudaMemcpyDeviceToHost, c.stream));
   CK(cudaStreamSynchronize(c.stream));
-  *total_out = total;
   if (ids && capacity >= total && total) {
-    QLAUNCH(true, offsets, ids);
+    uint32_t* d_ids = ids_host ? (uint32_t*)c.scratch.get(SLOT_FRONTIER_B, (size_t)total * 4) : ids;
+    if (!d_ids) return c.fail(OBVHS_ERR_OOM, "output staging");
+    QLAUNCH(true, offsets, d_ids);
     CK(cudaGetLastError());
+    if (ids_host) CK(cudaMemcpyAsync(ids, d_ids, (size_t)total * 4, cudaMemcpyDeviceToHost, c.stream));
   }
 #undef QLAUNCH
   return 0;
