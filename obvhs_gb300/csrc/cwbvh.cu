@@ -1558,6 +1558,9 @@ static const uint32_t* ceil_log2_thresholds() {
   return thr;
 }
 
+// A conversion that fails reports it itself: the next call starts without it.
+static void clear_status(BuildCtx& c) { cudaMemsetAsync(c.d_status, 0, 4, c.stream); }
+
 int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, int order_children, obvhs_cwbvh* out,
                          uint32_t* emitted_deferred, bool exact_aabbs, uint32_t ploc_passes, bool sound) {
   out->n_nodes = 0;
@@ -1616,8 +1619,10 @@ int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, i
   CK(cudaMemcpyAsync(&root, erec, sizeof(EmitRec), cudaMemcpyDeviceToHost, c.stream));
   CK(cudaMemcpyAsync(c.h_status, c.d_status, 4, cudaMemcpyDeviceToHost, c.stream));
   CK(cudaStreamSynchronize(c.stream));
-  if (*c.h_status)
+  if (*c.h_status) {
+    clear_status(c);
     return c.fail(OBVHS_ERR_BAD_INPUT, "BVH2 cannot be converted (a leaf holds more than one primitive)");
+  }
   const bool root_leaf = n == 1;
   if (root.z == OBVHS_INVALID)
     return c.fail(OBVHS_ERR_BAD_INPUT, "BVH2 cannot be converted (its links are not a tree's)");
@@ -1687,6 +1692,7 @@ int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, i
   CK(cudaMemcpyAsync(c.h_status, c.d_status, 4, cudaMemcpyDeviceToHost, c.stream));
   CK(cudaStreamSynchronize(c.stream));
   if (*c.h_status || emitted != n_cw) {
+    clear_status(c);
     cudaFree(cwn);
     cudaFree(cwp);
     if (exn) cudaFree(exn);
@@ -1750,8 +1756,10 @@ int cwbvh_seg_device(BuildCtx& c, const Bvh2Node* nodes, const uint32_t* pidx_in
   CK(cudaMemcpyAsync(hr.data(), roots, (size_t)S * sizeof(SegRoot), cudaMemcpyDeviceToHost, c.stream));
   CK(cudaMemcpyAsync(c.h_status, c.d_status, 4, cudaMemcpyDeviceToHost, c.stream));
   CK(cudaStreamSynchronize(c.stream));
-  if (*c.h_status)
+  if (*c.h_status) {
+    clear_status(c);
     return c.fail(OBVHS_ERR_BAD_INPUT, "BVH2 cannot be converted (a leaf holds more than one primitive)");
+  }
   // sizes, and one allocation for every scene's nodes, indices and triangles
   std::vector<uint32_t> n_cw(S), n_pr(S);
   std::vector<size_t> off(3 * (size_t)S);
