@@ -127,7 +127,8 @@ SIZES = [3, 40, 3000, 32_768, 40_000]
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", SIZES)
 @pytest.mark.parametrize("reinserted", [False, True])
-def test_nodes_of_no_tree_are_ignored(n, reinserted):
+@pytest.mark.parametrize("out_of_range", [False, True])
+def test_nodes_of_no_tree_are_ignored(n, reinserted, out_of_range):
     import obvhs_gb300 as G
 
     nodes, order, md = _tree(n, reinserted)
@@ -135,8 +136,9 @@ def test_nodes_of_no_tree_are_ignored(n, reinserted):
     pad = np.zeros((6, 32), np.uint8)
     ln = len(nodes)
     pad[:, :] = nodes[-1]  # a leaf ...
-    _word(pad, PRIMS)[:] = [1, 1, 0, 1, 0, 1]
-    _word(pad, FIRST)[:] = [0, 1, ln + 4, 0, ln + 20, 2]  # ... an inner node over two, one whose children are out of range
+    # ... an inner node over two of them, and perhaps one whose children are out of range
+    _word(pad, PRIMS)[:] = [1, 1, 0, 1, 0 if out_of_range else 1, 1]
+    _word(pad, FIRST)[:] = [0, 1, ln + 4, 0, ln + 20 if out_of_range else 1, 2]
     more = np.concatenate([nodes, pad])
     with G.Context() as ctx:
         # links of another tree in the context's scratch
