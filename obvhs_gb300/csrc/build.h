@@ -373,8 +373,8 @@ int reinsertion_device(BuildCtx& c, obvhs_bvh2* b, float batch_size_ratio, const
 // sets *unordered (zeroed by the caller) when some inner node's children are
 // not both at higher indices than the node.  With `odd` (zeroed by the caller,
 // `parents` filled with OBVHS_INVALID by it) the nodes may be any: nodes that
-// none names keep OBVHS_INVALID, and *odd is set where the links are not a
-// tree's.
+// none names keep OBVHS_INVALID, *odd is set where the links are not a tree's,
+// and *unordered where a child is out of range.
 int compute_parents_device(BuildCtx& c, const Bvh2Node* nodes, uint32_t n_nodes, uint32_t* parents,
                            uint32_t* unordered = nullptr, uint32_t* odd = nullptr);
 // Copies a host table to the device (stream-ordered, from pinned staging);

@@ -244,7 +244,7 @@ struct CostClimb {
       __stcg(&erec[i], make_uint4(0u, 0u, 1u, 0u));
       return false;
     }
-    if (p >= n) return false;  // (OBVHS_INVALID) a leaf that no node names: in no tree
+    if (p == OBVHS_INVALID) return false;  // a leaf that no node names: in no tree
     own = leaf_rec(nd);
     own_leaf = true;
     c = i;
@@ -286,7 +286,7 @@ struct CostClimb {
     own_list = list;
     own_leaf = false;
     __stcg(&erec[p], make_uint4(own.meta, aggn0, own.nprim, 0u));
-    if (up == p || up >= n) return true;  // a root, or the top of nodes that no tree names
+    if (up == p || up == OBVHS_INVALID) return true;  // a root, or the top of nodes that no tree names
     c = p;
     p = up;
     return false;
@@ -356,20 +356,7 @@ __device__ void costs_ordered(const Bvh2Node* __restrict__ nodes, const uint32_t
       continue;
     }
     const uint32_t f = node_first(nd);
-    if (f >= n_all - 1 || f < i) {
-      // an inert pad (children out of range).  A node above one, in a tree made
-      // elsewhere, has no finite distribution and too many primitives for a leaf
-      CostRec none;
-#pragma unroll
-      for (int k = 0; k < 7; k++) {
-        none.cost[k] = __int_as_float(0x7f800000);
-        none.contrib[k] = AGG_INVALID;
-      }
-      none.meta = 0;
-      none.nprim = 4;
-      st_rec(&crec[i], none);
-      __stcg(&erec[i], make_uint4(0u, AGG_INVALID, 4u, 0u));
-      __threadfence();
+    if (f + 1 >= n_all || f < i) {  // an inert pad (children out of range): nothing to compute
       atomicExch(&flags[i], 1u);
       continue;
     }
@@ -569,7 +556,7 @@ __device__ __forceinline__ uint32_t oct_bits(uint32_t ballot, int lane) { return
 // 4k nodes after reinsertion 95 -> 33 us, 20k nodes from PLOC (ready flags
 // polled level by level before) 120 -> 41 us.  The climb follows parent links, so
 // a launch that finds *odd set (links that are not a tree's) leaves the tree to
-// k_costs, which takes shared and unnamed nodes where they are in node order.
+// k_costs, which takes shared nodes where they are in node order.
 __global__ void __launch_bounds__(BLK) k_costs_oct(const Bvh2Node* __restrict__ nodes, const uint32_t* __restrict__ parents,
                                                    const uint32_t* __restrict__ pidx_in, uint32_t n, uint32_t max_prims,
                                                    CostRec* crec, EmitRec* erec, uint4* small, uint32_t* flags,
@@ -601,7 +588,7 @@ __global__ void __launch_bounds__(BLK) k_costs_oct(const Bvh2Node* __restrict__ 
         __stcg(&small[i], list);
         if (p == i) __stcg(&erec[i], make_uint4(0u, 0u, 1u, 0u));  // a leaf root: one CWBVH node
       }
-      if (p == i || p >= n) continue;  // a leaf root, or (OBVHS_INVALID) a leaf that no node names
+      if (p == i || p == OBVHS_INVALID) continue;  // a leaf root, or a leaf that no node names
       const CostRec r = leaf_rec(nd);
       cost = r.cost[0];
       contrib = 0;
@@ -733,7 +720,7 @@ __global__ void __launch_bounds__(BLK) k_costs_oct(const Bvh2Node* __restrict__ 
       meta = m;
       nprim = np;
       leaf = false;
-      climbing = up != p && up < n;
+      climbing = up != p && up != OBVHS_INVALID;
       c = p;
       p = up;
     }
@@ -1607,7 +1594,7 @@ int cwbvh_convert_device(BuildCtx& c, const obvhs_bvh2* b, uint32_t max_prims, i
     KLAUNCH("k_costs", CK(coop_launch(c, (const void*)k_costs_ranges, cost_range_grid(c), BLK, args, 0)));
   } else {
     CK(cudaMemsetAsync(flags, 0, flag_bytes, c.stream));
-    int r = compute_parents_device(c, b->nodes, n, parents, flags + n + 1);
+    int r = compute_parents_device(c, b->nodes, n, parents, flags + n + 1, sound ? nullptr : odd);
     if (r) return r;
     KLAUNCH("k_costs", launch_k(k_costs, cost_grid(c, n), BLK, 0, c.stream, b->nodes, parents, b->prim_indices, n,
                                 max_prims, crec, erec, small, flags, flags + n, flags + n + 1, c.d_status,

@@ -73,7 +73,9 @@ __global__ void k_parents(const Bvh2Node* __restrict__ nodes, uint32_t n, uint32
       parents[f + 1] = i;
     }
     if (odd && (!in_range || f == 0)) *odd = 1u;
-    if (unordered && in_range && f <= i) *unordered = 1u;
+    // (nothing climbs to a node with children out of range, the ordered pass would
+    // have to step over it)
+    if (unordered && (in_range ? f <= i : odd != nullptr)) *unordered = 1u;
   }
 }
 

@@ -192,6 +192,21 @@ def test_bad_links_are_an_error(n, reinserted, link):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [33_000, 65_537, 150_000, 400_000])
+def test_trees_in_node_order(n):
+    import obvhs_gb300 as G
+
+    nodes, order, md = _tree(n, False)
+    assert not _unordered(nodes)
+    want = O.bvh2_to_cwbvh(nodes, order, 3, True)
+    with G.Context() as ctx:
+        for _ in range(3):
+            got = _convert(G, ctx, nodes, order, md)
+            assert got[0].tobytes() == want[0].tobytes()
+            assert got[1].tobytes() == want[1].tobytes()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("link", [0, 1, INVALID])
 def test_inner_node_alone_is_an_error(link):
     import obvhs_gb300 as G
