@@ -68,8 +68,9 @@ __device__ __forceinline__ bool box_eq(const Box& a, const Box& b) {
 }
 
 // BVH2 node, 32 bytes: the field order of the reference's small_bvh2_node
-// layout (src/bvh2/node.rs:14-36): min, prim_count, max, first_index.
-struct __align__(16) Bvh2Node {
+// layout (src/bvh2/node.rs:14-36): min, prim_count, max, first_index.  Arrays
+// start on a 256-byte boundary; st_node writes a node in one 32-byte store.
+struct __align__(32) Bvh2Node {
   float4 a;  // min.xyz, prim_count (bits)
   float4 b;  // max.xyz, first_index (bits)
 };
@@ -100,7 +101,7 @@ __device__ __forceinline__ void st_256(void* p, const float4& a, const float4& b
                "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
                : "memory");
 }
-// Node arrays are allocations of their own, so every node is 32-byte aligned.
+static_assert(sizeof(Bvh2Node) == 32 && alignof(Bvh2Node) == 32, "st_256 writes aligned 32 bytes");
 __device__ __forceinline__ void st_node(Bvh2Node* p, const Bvh2Node& n) { st_256(p, n.a, n.b); }
 __device__ __forceinline__ Box node_box(const Bvh2Node& n) {
   return Box{make_float3(n.a.x, n.a.y, n.a.z), make_float3(n.b.x, n.b.y, n.b.z)};
