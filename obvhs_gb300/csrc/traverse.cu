@@ -226,7 +226,7 @@ __device__ __forceinline__ float intersect_ctri(const uint2* rec, float3 o, floa
 // slowest ray before taking new ones.
 constexpr uint32_t REFILL_IDLE = 4;
 
-// Persistent ray loop shared by the traversal kernels.  Each lane holds one
+// Persistent ray loop of the BVH2 traversal.  Each lane holds one
 // ray (`R`: start(ray index) sets it up and returns false when the ray is
 // already finished; step() advances it and returns true once it is finished;
 // both write the ray's result when it finishes) and runs its own loop.  A
@@ -234,35 +234,16 @@ constexpr uint32_t REFILL_IDLE = 4;
 // memory; once REFILL_IDLE lanes are idle the busy lanes leave their loops,
 // keeping their state, and the idle lanes take the next rays with one atomic
 // per warp.  The lanes converge only at the refill.
-//
-// `yield` (or null): the device's count of builds in flight, in mapped host
-// memory.  While it is non-zero, warps of odd blocks stop taking rays and
-// their blocks leave once their rays are done, so a concurrent build's
-// kernels find free slots on every SM instead of waiting for the whole
-// persistent grid; the even blocks take the remaining rays.  Lane 0 of a warp
-// of an odd block issues the read at every eighth refill and the warp acts on
-// the value at the next check, so the read is never waited for.
-template <class R, int TB = TBLK>
-__device__ __forceinline__ void persistent_rays(R& ray, uint32_t nrays, uint32_t* next_ray,
-                                                const uint32_t* yield = nullptr) {
+template <class R>
+__device__ __forceinline__ void persistent_rays(R& ray, uint32_t nrays, uint32_t* next_ray) {
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  __shared__ uint32_t s_idle[TB / 32];
+  __shared__ uint32_t s_idle[TBLK / 32];
   uint32_t* idle_ctr = &s_idle[threadIdx.x >> 5];
   bool alive = false;    // this lane holds a ray
   bool drained = false;  // (warp-uniform) the ray counter has run out
-  uint32_t refills = 0;
-  uint32_t yw = 0;  // lane 0: the count read at the last check
   for (;;) {
-    if (!drained && yield && (blockIdx.x & 1u)) {
-      uint32_t y = 0;
-      if (lane == 0 && (refills++ & 7u) == 0) {
-        y = yw;
-        asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(yw) : "l"(yield));
-      }
-      if (__shfl_sync(FULL, y, 0)) drained = true;
-    }
     if (!drained) {
       const uint32_t need = __ballot_sync(FULL, !alive);
       if (need) {
@@ -298,8 +279,9 @@ __device__ __forceinline__ void persistent_rays(R& ray, uint32_t nrays, uint32_t
   }
 }
 
-// Persistent ray loop for rays whose step comes in two kinds, a primitive
-// test and a node test (has_prim(), prim_step(), node_step()).  The warp
+// Persistent ray loop of the CWBVH traversals: `R` as above, but its step comes
+// in two kinds, a primitive test and a node test (has_prim(), prim_step(),
+// node_step()).  The warp
 // stays converged and takes one kind per iteration for the lanes that want
 // it: primitives as soon as at least a fifth of its rays wait with one, else
 // nodes.  A ray's own order of tests is untouched.  Letting each lane run to
@@ -308,11 +290,19 @@ __device__ __forceinline__ void persistent_rays(R& ray, uint32_t nrays, uint32_t
 // others go on with nodes.  Measured against that loop: 16M incoherent rays
 // on 8M triangles 15.81 -> 13.52 ms, 4M shadow rays on 2M 1868 -> 1633 us,
 // 2.07M primary rays on 1M 1627 -> 1600 us, 1M rays through a TLAS of 64
-// instances 549 -> 527 us.  Other thresholds (with a fused slab test: 13.33
-// ms / 1634 us / 1593 us at a fifth): half of the rays 14.93 ms / 1747 us /
-// 1883 us, any ray 18.06 ms / 1925 us / 1708 us.  Refill at 4 idle lanes
-// instead of 6 13.32 ms / 1631 us / 1594 us against 13.31 / 1613 / 1566, at 8
-// 13.47 / 1615 / 1556.
+// instances 549 -> 527 us.  Other thresholds (a fifth: 13.52 ms / 1638 us / 1611
+// us): an eighth of the rays 13.93 ms / 1679 us / 1602 us, a third 13.86 ms /
+// 1657 us / 1712 us, half 15.42 ms / 1779 us / 1924 us, any ray 16.69 ms / 1909
+// us / 1633 us.  Refill at 4 idle lanes instead of 6 13.52 ms / 1653 us / 1647
+// us, at 8 13.68 ms / 1641 us / 1610 us.
+//
+// `yield` (or null): the device's count of builds in flight, in mapped host
+// memory.  While it is non-zero, warps of odd blocks stop taking rays and
+// their blocks leave once their rays are done, so a concurrent build's
+// kernels find free slots on every SM instead of waiting for the whole
+// persistent grid; the even blocks take the remaining rays.  Lane 0 of a warp
+// of an odd block issues the read at every eighth refill and the warp acts on
+// the value at the next check, so the read is never waited for.
 constexpr int VOTED_REFILL_IDLE = 6;
 template <class R, int TB = TBLK>
 __device__ __forceinline__ void voted_rays(R& ray, uint32_t nrays, uint32_t* next_ray, const uint32_t* yield,
@@ -370,8 +360,8 @@ __device__ __forceinline__ void voted_rays(R& ray, uint32_t nrays, uint32_t* nex
 // as RtCompressedTriangle (24 B; the hit's original id comes from
 // primitive_indices) instead of the 64-byte records.  MULTI: every ray names
 // its BVH (ray_bvh[ray] indexes `multi`), so ray batches against different
-// BVHs run in one launch.  A step handles the primitives of the current
-// group, then pops one child node (or a group from the stack).
+// BVHs run in one launch.  A step tests one primitive or one child node of the
+// current group; a group with neither left gives way to the next on the stack.
 template <int MODE, bool CTRI, bool MULTI, int STRIDE = 1>
 struct CwRay {
   // launch inputs
