@@ -133,6 +133,18 @@ struct __align__(16) CwNode {
   uint4 q[5];
 };
 
+// The valid lanes of the warp with this lane's 8-bit digit, by a ballot per bit
+// (meaningless in a lane that is not valid; all 32 lanes take part).
+__device__ __forceinline__ uint32_t same_digit_lanes(uint32_t d, bool valid) {
+  uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    const uint32_t bit = (uint32_t)((int32_t)(d << (31 - b)) >> 31);  // all ones or zeros
+    peers &= ~(__ballot_sync(0xffffffffu, bit != 0u) ^ bit);
+  }
+  return peers;
+}
+
 template <class T>
 __host__ __device__ __forceinline__ T div_up(T a, T b) {
   return (a + b - 1) / b;

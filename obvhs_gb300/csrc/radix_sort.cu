@@ -154,12 +154,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_rs_pass(const K* __restrict__ ke
     const uint32_t i = wbase + r * 32 + lane;
     const bool valid = i < n;
     const uint32_t d = valid ? KeyTraits<K>::digit(key[r], byte) : 256u;
-    uint32_t peers = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-    for (int b = 0; b < 8; b++) {
-      const uint32_t bit = (uint32_t)((int32_t)(d << (31 - b)) >> 31);  // all ones or zeros
-      peers &= ~(__ballot_sync(0xffffffffu, bit != 0u) ^ bit);
-    }
+    const uint32_t peers = same_digit_lanes(d, valid);
     const uint32_t lrank = __popc(peers & lt_mask);
     const uint32_t before = valid ? wh[d] : 0u;
     __syncwarp();

@@ -157,7 +157,9 @@ __global__ void __launch_bounds__(BLK) k_cand_keys(const Bvh2Node* __restrict__ 
 // the block's barriers and the ballot / shared-memory chain of a digit pass (in a
 // batch of 96 scenes 31.8 us a launch, 39.1 with match.any in place of the
 // ballots); a batch runs as many blocks as scenes.  96 scenes of 1k-200k
-// triangles 7432 -> 7010 us, then 5612 -> 5573 with the ballots.  (For one tree a
+// triangles 7432 -> 7010 us, then 5612 -> 5573 with the ballots; against the
+// global sort with its ballots 5707 -> 5573 us, 8 of 30k-60k (fast) 1543 -> 1519,
+// two of 60k even.  (For one tree a
 // block takes longer than the global sort above 8,000 candidates: 100k
 // triangles, slow build, 2789 -> 2894 us.)  A thread keeps up to CS_ITEMS
 // candidates in registers; warp w owns the contiguous candidates [w * 32 * I,
@@ -238,12 +240,7 @@ __device__ __forceinline__ void sort_candidates(const Bvh2Node* nodes, uint32_t 
       if ((uint32_t)r >= items) break;
       const bool valid = base_i + 32u * r < n;
       const uint32_t d = valid ? (key[r] >> shift) & 0xffu : 256u;
-      uint32_t peers = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-      for (int b = 0; b < 8; b++) {  // as in the radix passes: cheaper than match.any
-        const uint32_t bit = (uint32_t)((int32_t)(d << (31 - b)) >> 31);
-        peers &= ~(__ballot_sync(0xffffffffu, bit != 0u) ^ bit);
-      }
+      const uint32_t peers = same_digit_lanes(d, valid);
       const uint32_t lrank = __popc(peers & lt_mask);
       const uint32_t before = valid ? wh[d] : 0u;
       __syncwarp();
@@ -616,10 +613,14 @@ __global__ void __launch_bounds__(FIND_THREADS) k_find_persistent(const Bvh2Node
 // dependent loads.  Builds: 100k triangles, medium, 1747 -> 1413 us; 30k 1256
 // -> 942; 300k 2572 -> 2280; 100k, slow, 2789 -> 2528; 20 scenes of 2k-50k 2977
 // -> 2451 us.
-// The line at RF_MAX: with 8,192 instead the 300k build takes 2344 us, with
-// 4,096 2419; above 16,384 the keys leave room for two blocks an SM and the
+// The line at RF_MAX: the 300k medium build takes 2242 us, with 12,288 instead
+// 2244, with 8,192 2252, with 4,096 2315; the 100k slow build 2500, 2501, 2512,
+// 2608; above 16,384 the keys leave room for two blocks an SM and the
 // comparisons grow past the sort's time.  RF_PAIRS, the comparisons of a batch's
-// launch: 64M keeps 96 scenes at 7028 us; 256M 7086, 1,024M 7206.
+// launch, above which its scenes' candidates are sorted by a block each: with
+// 16M / 64M / 256M / 1,024M 96 scenes take 5587 / 5573 / 5635 / 5759 us, 20 of
+// 2k-50k 1866 / 1850 / 1887 / 1886, three of 40k-100k (slow) 2555 / 2486 / 2456 /
+// 2448.
 constexpr int RF_THREADS = 512;
 constexpr uint32_t RF_CAND = 64;
 constexpr uint32_t RF_SLICES = RF_THREADS / RF_CAND;
