@@ -356,7 +356,11 @@ __device__ void costs_ordered(const Bvh2Node* __restrict__ nodes, const uint32_t
       continue;
     }
     const uint32_t f = node_first(nd);
-    if (f + 1 >= n_all || f < i) {  // an inert pad (children out of range): nothing to compute
+    // an inert pad of a segmented build (children out of range): nothing to
+    // compute.  (Trees made elsewhere come here with every child in range.  As
+    // f >= n_all - 1 the test took sound nodes of trees above 65,000 nodes for pads:
+    // ptxas 13.0 at -O3, not at -O1)
+    if (f + 1 >= n_all || f < i) {
       atomicExch(&flags[i], 1u);
       continue;
     }
