@@ -131,7 +131,8 @@ class Context:
     def set_traversal_config(self, block: int = 0, smem_stack: bool = False):
         """Launch form of this context's CWBVH traversals: block size and
         where each ray's 32-entry group stack lives (identical results in
-        every form; (0, False) is the default (128, local memory))."""
+        every form; (0, False) is the default (128, local memory), in which a
+        call of few rays gives each warp fewer than 32 of them)."""
         self.check(self.lib.obvhs_ctx_set_traversal_config(self.h, int(block), int(bool(smem_stack))))
 
     #: OBVHS_DEFAULT_WAIT_LIMIT in include/obvhs_gb300.h
